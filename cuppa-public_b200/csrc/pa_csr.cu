@@ -78,10 +78,10 @@ __global__ void seed_out_kernel(uint32_t d, uint32_t seed_mode, uint32_t *seed_o
 //
 // A pass sorts 8 or 9 key bits (the fewest passes for the key).  Its
 // kernel claims tiles of 8192 items in order from a counter; a tile's 512
-// threads load 16 items each and park them in shared memory, rank them stably
-// -- each of 16 warps walks its 512 items in order, 32 at a time, with
-// __match_any_sync for equal digits and 16-bit per-warp counters in shared
-// memory -- publish the tile's count of every digit, and look back over the
+// threads take 16 items each and rank them stably -- each of 16 warps walks its
+// 512 items in order, 32 at a time; a digit's word in shared memory collects the
+// round's lanes that hold it (atomicOr) beside its count so far -- publish the
+// tile's count of every digit, and look back over the
 // tiles before it (their counts, or the running total the nearest finished
 // one published) for each digit's global offset.  The tile is then staged in
 // shared memory in digit order and every digit's run is written contiguously.
@@ -174,23 +174,36 @@ __global__ void radix_base_kernel(const unsigned long long *hist, uint32_t passe
     }
 }
 
-// Dynamic shared memory of the pass kernel: the tile in digit order, each
-// digit's global offset less its start within the tile, the per-warp digit
-// counts (then the warps' bases within the tile), the claimed tile.
+// Dynamic shared memory of the pass kernel: the warps' digit words while the
+// tile is ranked, then the tile in digit order in their place; each digit's
+// global offset less its start within the tile, the warps' bases within the
+// tile, the claimed tile.
 template <uint32_t NB>
 struct RadixSmem {
-    unsigned long long stage[kRadixTile];
+    union {
+        unsigned long long stage[kRadixTile];
+        uint2 word[kRadixWarps][NB];   // x: lanes of this round holding the digit, y: count so far
+    };
     unsigned long long goff[NB];
     uint16_t wcnt[kRadixWarps][NB];
     uint32_t wsum[kRadixWarps];
     unsigned long long tile;
 };
 
-// Two CTAs per SM (84 KB of shared memory each at 9-bit digits, 64 registers).
-// Measured at n = 2^30, d = 4 (C3 CSR) and n = 10^8, d = 16 (C2): 8,192-item
-// tiles at two CTAs 224-227 / 75.6 ms; 6,144-item tiles at three CTAs and 40
-// registers (which spill) 231 / 76.0 ms; 7,168, 9,216 and 10,240-item tiles at
-// two CTAs 231 / 74.2, 238 / 76.8 and 241 / 77.1 ms.
+// What bounds it: the shared-memory pipe (77 % busy in a capture at 9.6 * 10^7
+// items; DRAM 27 %), ~52 wavefronts per 32 items.  __match_any_sync for the
+// equal digits, which the words replace, costs two cycles of a unit shared by
+// the SM per distinct value: 61 cycles a round of 32 mostly distinct digits
+// against 7.5 for the atomicOr, the word's load and its store (measured alone).
+// n = 2.5 * 10^7, d = 16 (4 * 10^8 items): the CSR build 17.7 -> 15.1 ms, a pass
+// 3.9 -> 2.95 ms.  Holding the items in registers instead of reading them a
+// second time spills and measured the same (15.1 ms).
+//
+// Two CTAs per SM (86 KB of shared memory each at 9-bit digits, 64 registers).
+// With the earlier ranking, at n = 2^30, d = 4 (C3 CSR) and n = 10^8, d = 16
+// (C2): 8,192-item tiles at two CTAs 224-227 / 75.6 ms; 6,144-item tiles at three
+// CTAs and 40 registers (which spill) 231 / 76.0 ms; 7,168, 9,216 and
+// 10,240-item tiles at two CTAs 231 / 74.2, 238 / 76.8 and 241 / 77.1 ms.
 template <uint32_t DB>
 __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(
     const unsigned long long *src, unsigned long long *dst, uint64_t n_items, uint32_t shift,
@@ -206,59 +219,48 @@ __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t lt = lanemask_lt();
     const bool owner = tid * DPT < NB;
-    for (uint32_t w = 0; w < kRadixWarps; ++w)
-        for (uint32_t b = tid; b < NB; b += kRadixThreads) S.wcnt[w][b] = 0;
     if (tid == 0) S.tile = atomicAdd(tile_ctr, 1ull);
+    for (uint32_t b = lane; b < NB; b += 32) S.word[warp][b] = make_uint2(0u, 0u);
     __syncthreads();
     const uint64_t t = S.tile;
     const uint64_t tb = t * kRadixTile;
     const uint32_t tcount = (uint32_t)min((uint64_t)kRadixTile, n_items - tb);
     const uint32_t wo = warp * (kRadixRounds * 32);
 
-    // 1. the tile's items, loaded together, parked in the stage in their own
-    // order (conflict-free); only their digits stay in registers through the
-    // ranking and the look-back, which keeps the kernel free of spills
+    // 1. the digits of the tile's items (the keys, the items' high words), all
+    // loads in flight together; the items themselves are read again for the
+    // staging, from L2
     uint32_t dgp[kRadixRounds / 2];   // two digits per register
-    // loaded in two halves: all of a thread's items at once spill registers
+    {
+        const uint32_t *key = reinterpret_cast<const uint32_t *>(src + tb) + 1;
+        uint32_t kv[kRadixRounds];
 #pragma unroll
-    for (uint32_t h = 0; h < kRadixRounds; h += kRadixRounds / 2) {
-        unsigned long long its[kRadixRounds / 2];
-#pragma unroll
-        for (uint32_t q = 0; q < kRadixRounds / 2; ++q) {
-            const uint32_t k = wo + (h + q) * 32 + lane;
-            its[q] = k < tcount ? src[tb + k] : 0ull;
-        }
-#pragma unroll
-        for (uint32_t q = 0; q < kRadixRounds / 2; ++q) {
-            const uint32_t r = h + q;
+        for (uint32_t r = 0; r < kRadixRounds; ++r) {
             const uint32_t k = wo + r * 32 + lane;
-            S.stage[k] = its[q];
-            const uint32_t dg = k < tcount ? (uint32_t)(its[q] >> (32 + shift)) & MASK : NB + lane;
-            if (r & 1) dgp[r / 2] |= dg << 16;
-            else dgp[r / 2] = dg;
+            kv[r] = k < tcount ? key[2 * k] : 0u;
         }
+#pragma unroll
+        for (uint32_t r = 0; r < kRadixRounds; r += 2)
+            dgp[r / 2] = ((kv[r] >> shift) & MASK) | (((kv[r + 1] >> shift) & MASK) << 16);
     }
     // stable ranks within the warp's items (in order, 32 per round); two ranks
     // per register
     uint32_t rk[kRadixRounds / 2];
+    uint2 *const word = S.word[warp];
 #pragma unroll
     for (uint32_t r = 0; r < kRadixRounds; ++r) {
-        const uint32_t k = wo + r * 32 + lane;
-        const bool valid = k < tcount;
+        const bool valid = wo + r * 32 + lane < tcount;
         const uint32_t dg = (dgp[r / 2] >> ((r & 1) * 16)) & 0xffffu;
-        const uint32_t peers = __match_any_sync(kFull, dg);
-        const uint32_t leader = __ffs(peers) - 1;
-        uint32_t old = 0;
-        if (valid && lane == leader) {
-            old = S.wcnt[warp][dg];
-            S.wcnt[warp][dg] = (uint16_t)(old + __popc(peers));
-        }
-        old = __shfl_sync(kFull, old, leader);
-        const uint32_t rank = old + __popc(peers & lt);
+        if (valid) atomicOr(&word[dg].x, 1u << lane);
+        __syncwarp();
+        uint2 w = make_uint2(0u, 0u);
+        if (valid) w = word[dg];
+        // every lane has read its word before its lowest lane clears the mask
+        __syncwarp();
+        if (valid && (w.x & lt) == 0u) word[dg] = make_uint2(0u, w.y + __popc(w.x));
+        const uint32_t rank = w.y + __popc(w.x & lt);
         if (r & 1) rk[r / 2] |= rank << 16;
         else rk[r / 2] = rank;
-        // the next round's leader for a digit may be another lane: order this
-        // round's counter stores before the next round's loads
         __syncwarp();
     }
     __syncthreads();
@@ -271,8 +273,9 @@ __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(
         tot[j] = 0;
         if (owner) {
             const uint32_t dig = tid * DPT + j;
+#pragma unroll
             for (uint32_t w = 0; w < kRadixWarps; ++w) {
-                const uint32_t c = S.wcnt[w][dig];
+                const uint32_t c = S.word[w][dig].y;
                 S.wcnt[w][dig] = (uint16_t)tot[j];
                 tot[j] += c;
             }
@@ -376,19 +379,23 @@ __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(
         }
     }
     __syncthreads();
-    // 5. the tile back from its parking place, then into the stage in digit order
-    {
-        unsigned long long its[kRadixRounds];
+    // 5. the tile's items (read a second time) into the stage in digit order;
+    // the words under the stage were last read before the barrier above
 #pragma unroll
-        for (uint32_t r = 0; r < kRadixRounds; ++r) its[r] = S.stage[wo + r * 32 + lane];
-        __syncthreads();
+    for (uint32_t h = 0; h < kRadixRounds; h += kRadixRounds / 2) {
+        unsigned long long its[kRadixRounds / 2];
 #pragma unroll
-        for (uint32_t r = 0; r < kRadixRounds; ++r) {
-            const uint32_t k = wo + r * 32 + lane;
-            if (k < tcount) {
+        for (uint32_t q = 0; q < kRadixRounds / 2; ++q) {
+            const uint32_t k = wo + (h + q) * 32 + lane;
+            its[q] = k < tcount ? src[tb + k] : 0ull;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kRadixRounds / 2; ++q) {
+            const uint32_t r = h + q;
+            if (wo + r * 32 + lane < tcount) {
                 const uint32_t dg = (dgp[r / 2] >> ((r & 1) * 16)) & 0xffffu;
                 const uint32_t rank = (rk[r / 2] >> ((r & 1) * 16)) & 0xffffu;
-                S.stage[S.wcnt[warp][dg] + rank] = its[r];
+                S.stage[S.wcnt[warp][dg] + rank] = its[q];
             }
         }
     }
