@@ -55,58 +55,138 @@ __global__ void canon_kernel(const Id *in, Id *out, uint64_t n, uint32_t d, uint
     }
 }
 
-// Undirected degree: +1 on both endpoints of every pair.  Equal endpoints in a
-// warp are combined with __match_any_sync before the atomic (hub nodes take
-// most increments when p is small).
-template <typename Id>
-__global__ void degree_kernel(const Id *E, uint64_t n_edges, uint64_t n, unsigned long long *deg)
+// ---------------------------------------------------------------------------
+// Undirected degrees.
+//
+// A generated pair's source is known from its place (pair seed_edges + r*d + j
+// belongs to node u_first + r), so the counts start at d for every generated node
+// and a pair costs one atomic, for its target; a pair whose source is another
+// (a list in some other order) moves one count from the expected node to its own.
+//
+// What bounds it: the target atomics, spread over the whole count array.  They
+// run at L2 speed only while the array stays in L2, so the counts are 32 bits
+// wide, in the front half of the output, and widened in place at the end
+// (64-bit counts for lists of 2^31 pairs and more, and below kDegNarrow nodes,
+// whose 64-bit counts are in L2 too and need no widening launches).  Early nodes hold the
+// hubs: ids below kLowIds are counted in shared memory, one flush per block.
+// n = 2^24, d = 8, p = 0.3, 32-bit ids: 5.63 -> 0.97 ms (138 G targets/s; two
+// atomics a pair combined by __match_any_sync before); p = 0.1, 64-bit ids:
+// 15.9 -> 0.82 ms; n = 10^6: 0.309 -> 0.062 ms.
+// ---------------------------------------------------------------------------
+constexpr uint32_t kDegThreads = 512;
+constexpr uint32_t kDegChunk = 8192;   // pairs per block step at most
+constexpr uint64_t kDegNarrow = 1ull << 22;   // nodes above which 32-bit counts pay
+constexpr uint32_t kLowIds = 8192;     // 32 KB of shared counters
+
+template <typename Cnt>
+__global__ void __launch_bounds__(kDegThreads) degree_init_kernel(Cnt *deg, uint64_t n, uint64_t u_first,
+                                                                  uint32_t d)
 {
-    const uint32_t lane = threadIdx.x & 31u;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n_edges; base += stride) {
-        const uint64_t e = base + threadIdx.x;
-        unsigned long long s = e < n_edges ? (unsigned long long)E[2 * e] : ~0ull;
-        unsigned long long t = e < n_edges ? (unsigned long long)E[2 * e + 1] : ~0ull;
-        const bool act = s < n && t < n;   // ids are used as addresses: never trust them
-        if (!act) s = t = ~0ull - lane;    // unique keys, never a leader for a real id
-        const uint32_t ms = __match_any_sync(kFull, s);
-        const uint32_t mt = __match_any_sync(kFull, t);
-        if (act && (__ffs(ms) - 1) == (int)lane) atomicAdd(deg + s, (unsigned long long)__popc(ms));
-        if (act && (__ffs(mt) - 1) == (int)lane) atomicAdd(deg + t, (unsigned long long)__popc(mt));
-    }
+    for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += stride)
+        deg[u] = u >= u_first ? (Cnt)d : (Cnt)0;
 }
 
-// The same over a SLOTS graph: a group of d lanes takes one row (node
-// u_first + row, targets S[row*d ..]); the seed edges come from their closed form.
-template <typename Id>
-__global__ void degree_slots_kernel(const Id *S, uint64_t rows, uint32_t d, uint64_t u_first,
-                                    uint32_t seed_mode, uint64_t seed_edges, uint64_t n,
-                                    unsigned long long *deg)
+// Pairs (or, with Slots, targets) of the generated nodes: `count` of them from E
+// + (Slots ? 0 : 2) * seed_edges, `chunk` (<= kDegChunk) a block step; block 0 also
+// counts the seed edges.
+template <typename Id, bool Slots, typename Cnt>
+__global__ void __launch_bounds__(kDegThreads) degree_kernel(const Id *E, uint64_t count,
+                                                             uint32_t chunk, uint32_t d,
+                                                             uint32_t d_inv, uint64_t u_first,
+                                                             uint32_t seed_mode, uint64_t seed_edges,
+                                                             uint64_t n, bool vec, Cnt *deg)
 {
-    const uint32_t lane = threadIdx.x & 31u;
-    const uint32_t G = 32u / d;
-    const uint32_t g = lane / d;
-    const bool used = lane < G * d;
-    const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
-    const uint64_t w0 = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    if (w0 == 0)
-        for (uint64_t e = lane; e < seed_edges; e += 32) {
+    __shared__ uint32_t low[kLowIds];
+    for (uint32_t i = threadIdx.x; i < kLowIds; i += kDegThreads) low[i] = 0;
+    __syncthreads();
+    if (blockIdx.x == 0)
+        for (uint64_t e = threadIdx.x; e < seed_edges; e += kDegThreads) {
             uint64_t s, t;
-            seed_edge_of(e, d, seed_mode, s, t);
-            atomicAdd(deg + s, 1ull);
-            atomicAdd(deg + t, 1ull);
+            if constexpr (Slots) {
+                seed_edge_of(e, d, seed_mode, s, t);
+            } else {
+                s = (uint64_t)E[2 * e];
+                t = (uint64_t)E[2 * e + 1];
+            }
+            if (s < n && t < n) {   // ids are used as addresses: never trust them
+                atomicAdd(deg + s, (Cnt)1);
+                atomicAdd(deg + t, (Cnt)1);
+            }
         }
-    for (uint64_t r0 = w0 * G; r0 < rows; r0 += warps * G) {
-        const uint64_t row = r0 + g;
-        const bool in = used && row < rows;
-        unsigned long long t = in ? (unsigned long long)S[row * d + (lane - g * d)] : ~0ull;
-        const bool act = in && t < n;       // ids are used as addresses: never trust them
-        if (!act) t = ~0ull - lane;
-        const uint32_t mt = __match_any_sync(kFull, t);
-        if (act && (__ffs(mt) - 1) == (int)lane) atomicAdd(deg + t, (unsigned long long)__popc(mt));
-        // the row's own node: d increments, from its first lane
-        if (in && lane == g * d) atomicAdd(deg + u_first + row, (unsigned long long)d);
+    const Id *G = E + (Slots ? 0 : 2 * seed_edges);
+    constexpr uint32_t U = 4;   // loads in flight per thread
+    for (uint64_t c0 = (uint64_t)blockIdx.x * chunk; c0 < count; c0 += (uint64_t)gridDim.x * chunk) {
+        const uint64_t row0 = c0 / d;
+        const uint32_t x0 = (uint32_t)(c0 - row0 * d);   // the chunk starts at slot x0 of row row0
+        const uint32_t len = (uint32_t)min((uint64_t)chunk, count - c0);
+        for (uint32_t b = threadIdx.x; b < len; b += U * kDegThreads) {
+            uint64_t s[U], t[U];
+#pragma unroll
+            for (uint32_t q = 0; q < U; ++q) {
+                const uint32_t x = b + q * kDegThreads;
+                t[q] = ~0ull;
+                s[q] = ~0ull;
+                if (x < len) {
+                    if constexpr (Slots) {
+                        t[q] = (uint64_t)__ldcs(G + c0 + x);
+                    } else if (!vec) {
+                        s[q] = (uint64_t)(int64_t)G[2 * (c0 + x)];
+                        t[q] = (uint64_t)(int64_t)G[2 * (c0 + x) + 1];
+                    } else if constexpr (sizeof(Id) == 4) {
+                        const int2 w = __ldcs(reinterpret_cast<const int2 *>(G) + c0 + x);
+                        s[q] = (uint64_t)(int64_t)w.x;
+                        t[q] = (uint64_t)(int64_t)w.y;
+                    } else {
+                        const longlong2 w = __ldcs(reinterpret_cast<const longlong2 *>(G) + c0 + x);
+                        s[q] = (uint64_t)w.x;
+                        t[q] = (uint64_t)w.y;
+                    }
+                }
+            }
+#pragma unroll
+            for (uint32_t q = 0; q < U; ++q) {
+                const uint32_t x = b + q * kDegThreads;
+                if (x >= len) continue;
+                if (Slots ? t[q] < n : (t[q] < n && s[q] < n)) {
+                    if (t[q] < kLowIds) atomicAdd(low + t[q], 1u);
+                    else atomicAdd(deg + t[q], (Cnt)1);
+                } else {
+                    t[q] = ~0ull;   // not counted at either end
+                }
+                if constexpr (!Slots) {
+                    const uint64_t u = u_first + row0 + (d == 1 ? x : __umulhi(x0 + x, d_inv));
+                    if (s[q] != u || t[q] == ~0ull) {
+                        atomicAdd(deg + u, (Cnt)-1);
+                        if (t[q] != ~0ull) atomicAdd(deg + s[q], (Cnt)1);
+                    }
+                }
+            }
+        }
     }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < kLowIds; i += kDegThreads)
+        if (low[i]) atomicAdd(deg + i, (Cnt)low[i]);   // ids below n only were counted
+}
+
+// 32-bit counts [lo, hi) of the array's front to 64 bits in place: 8 lo >= 4 hi,
+// so no count of the range is overwritten before it is read.
+__global__ void __launch_bounds__(256) widen_kernel(uint32_t *c, uint64_t lo, uint64_t hi)
+{
+    unsigned long long *w = reinterpret_cast<unsigned long long *>(c);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = lo + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < hi; i += stride)
+        w[i] = c[i];
+}
+
+// The first `count` (at most kLowIds) of them, through shared memory (one block).
+__global__ void __launch_bounds__(1024) widen_low_kernel(uint32_t *c, uint32_t count)
+{
+    __shared__ uint32_t v[kLowIds];
+    for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) v[i] = c[i];
+    __syncthreads();
+    unsigned long long *w = reinterpret_cast<unsigned long long *>(c);
+    for (uint32_t i = threadIdx.x; i < count; i += blockDim.x) w[i] = v[i];
 }
 
 // MurmurHash3's 64-bit finalizer (Appleby, public domain): a bijective mix.
@@ -178,37 +258,53 @@ __global__ void __launch_bounds__(256) digest_kernel(const Id *x, uint64_t count
     }
 }
 
-// The same for d > 32: one thread per slot (slot j of row j / d); the row's
-// node gets its d increments from the thread of the row's first slot.
-template <typename Id>
-__global__ void degree_slots_any_kernel(const Id *S, uint64_t rows, uint32_t d, uint64_t u_first,
-                                        uint32_t seed_mode, uint64_t seed_edges, uint64_t n,
-                                        unsigned long long *deg)
-{
-    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const uint64_t t0 = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    for (uint64_t e = t0; e < seed_edges; e += stride) {
-        uint64_t s, t;
-        seed_edge_of(e, d, seed_mode, s, t);
-        atomicAdd(deg + s, 1ull);
-        atomicAdd(deg + t, 1ull);
-    }
-    for (uint64_t j = t0; j < rows * d; j += stride) {
-        const unsigned long long t = (unsigned long long)S[j];
-        if (t < n) atomicAdd(deg + t, 1ull);   // ids are used as addresses: never trust them
-        if (j % d == 0) atomicAdd(deg + u_first + j / d, (unsigned long long)d);
-    }
-}
-
-int grid_for(uint64_t work_items, uint32_t threads)
+int grid_for(uint64_t work_items, uint32_t threads, uint32_t per_sm = 8)
 {
     int dev = 0, sms = 148;
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
     uint64_t want = (work_items + threads - 1) / threads;
-    const uint64_t cap = (uint64_t)sms * 8;
+    const uint64_t cap = (uint64_t)sms * per_sm;
     if (want > cap) want = cap;
     return (int)(want ? want : 1);
+}
+
+template <typename Id, bool Slots, typename Cnt>
+void degrees_launch(const pa_params *prm, const GenPlan &p, const Id *E, Cnt *deg, cudaStream_t s)
+{
+    const uint64_t n = prm->n, count = (n - p.u_first) * prm->d;
+    degree_init_kernel<Cnt><<<grid_for(n, kDegThreads), kDegThreads, 0, s>>>(deg, n, p.u_first, prm->d);
+    // floor(x / d) = umulhi(x, d_inv) for x below 2^16: d_inv = ceil(2^32 / d) is off
+    // by less than 1 / x (d = 1: 2^32 does not fit)
+    // one load per pair when the pairs are aligned to their size
+    const bool vec = (reinterpret_cast<uintptr_t>(E) & (2 * sizeof(Id) - 1)) == 0;
+    const uint32_t d_inv = (uint32_t)(((1ull << 32) + prm->d - 1) / prm->d);
+    // whole chunks, four blocks per SM; less per block step where that leaves SMs idle
+    uint32_t chunk = kDegChunk;
+    while (chunk > 1024 && count < 600ull * chunk) chunk /= 2;
+    degree_kernel<Id, Slots, Cnt><<<grid_for(count, chunk, 4), kDegThreads, 0, s>>>(
+        E, count, chunk, prm->d, d_inv, p.u_first, prm->seed_mode, p.seed_edges, n, vec, deg);
+}
+
+template <typename Id>
+void degrees_any(const pa_params *prm, const GenPlan &p, const Id *E, int64_t *d_deg, cudaStream_t s)
+{
+    if (p.n_edges >= (1ull << 31) || prm->n <= kDegNarrow) {
+        unsigned long long *deg = reinterpret_cast<unsigned long long *>(d_deg);
+        if (p.slots) degrees_launch<Id, true>(prm, p, E, deg, s);
+        else degrees_launch<Id, false>(prm, p, E, deg, s);
+        return;
+    }
+    uint32_t *deg = reinterpret_cast<uint32_t *>(d_deg);
+    if (p.slots) degrees_launch<Id, true>(prm, p, E, deg, s);
+    else degrees_launch<Id, false>(prm, p, E, deg, s);
+    uint64_t hi = prm->n;
+    while (hi > kLowIds) {
+        const uint64_t lo = (hi + 1) / 2;
+        widen_kernel<<<grid_for(hi - lo, 256), 256, 0, s>>>(deg, lo, hi);
+        hi = lo;
+    }
+    widen_low_kernel<<<1, 1024, 0, s>>>(deg, (uint32_t)hi);
 }
 
 }  // namespace
@@ -247,39 +343,9 @@ int pa_degrees(const pa_params *prm, const void *d_edges, int64_t *d_deg, void *
     if (rc != PA_OK) return rc;
     if (!d_edges || !d_deg) return PA_ERR_INVALID;
     cudaStream_t s = (cudaStream_t)stream;
-    cudaError_t e = cudaMemsetAsync(d_deg, 0, prm->n * sizeof(int64_t), s);
-    if (e != cudaSuccess) return set_cuda_error(e);
-    const uint32_t threads = 256;
-    const int grid = grid_for(p.n_edges, threads);
-    if (p.slots && p.wide) {
-        const uint64_t rows = prm->n - p.u_first;
-        if (p.id_bytes == 8)
-            degree_slots_any_kernel<int64_t><<<grid, threads, 0, s>>>(
-                (const int64_t *)d_edges, rows, prm->d, p.u_first, prm->seed_mode, p.seed_edges,
-                prm->n, (unsigned long long *)d_deg);
-        else
-            degree_slots_any_kernel<int32_t><<<grid, threads, 0, s>>>(
-                (const int32_t *)d_edges, rows, prm->d, p.u_first, prm->seed_mode, p.seed_edges,
-                prm->n, (unsigned long long *)d_deg);
-    } else if (p.slots) {
-        const uint64_t rows = prm->n - p.u_first;
-        if (p.id_bytes == 8)
-            degree_slots_kernel<int64_t><<<grid, threads, 0, s>>>(
-                (const int64_t *)d_edges, rows, prm->d, p.u_first, prm->seed_mode, p.seed_edges,
-                prm->n, (unsigned long long *)d_deg);
-        else
-            degree_slots_kernel<int32_t><<<grid, threads, 0, s>>>(
-                (const int32_t *)d_edges, rows, prm->d, p.u_first, prm->seed_mode, p.seed_edges,
-                prm->n, (unsigned long long *)d_deg);
-    } else if (p.n_edges) {
-        if (p.id_bytes == 8)
-            degree_kernel<int64_t><<<grid, threads, 0, s>>>((const int64_t *)d_edges, p.n_edges,
-                                                            prm->n, (unsigned long long *)d_deg);
-        else
-            degree_kernel<int32_t><<<grid, threads, 0, s>>>((const int32_t *)d_edges, p.n_edges,
-                                                            prm->n, (unsigned long long *)d_deg);
-    }
-    e = cudaGetLastError();
+    if (p.id_bytes == 8) degrees_any<int64_t>(prm, p, (const int64_t *)d_edges, d_deg, s);
+    else degrees_any<int32_t>(prm, p, (const int32_t *)d_edges, d_deg, s);
+    const cudaError_t e = cudaGetLastError();
     return e == cudaSuccess ? PA_OK : set_cuda_error(e);
 }
 
