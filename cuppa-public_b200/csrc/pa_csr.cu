@@ -56,14 +56,6 @@ __global__ void seed_out_part_kernel(const Id *E, const int64_t *rowptr, Id *col
     }
 }
 
-// Out-degree of each seed node: CLIQUE row v holds v edges (to 0..v-1),
-// STAR_REF node d holds d (to 0..d-1).
-__global__ void seed_out_kernel(uint32_t d, uint32_t seed_mode, uint32_t *seed_out)
-{
-    for (uint32_t v = threadIdx.x; v <= d; v += blockDim.x)
-        seed_out[v] = seed_mode == PA_SEED_CLIQUE ? v : (v == d ? d : 0u);
-}
-
 // ---------------------------------------------------------------------------
 // Sorted in parts by a stable LSD radix sort (graphs below 2^32 nodes).
 //
@@ -88,9 +80,11 @@ __global__ void seed_out_kernel(uint32_t d, uint32_t seed_mode, uint32_t *seed_o
 // ---------------------------------------------------------------------------
 constexpr uint32_t kRadixThreads = 512, kRadixWarps = kRadixThreads / 32;
 constexpr uint32_t kRadixBuckets = 512;   // the widest digit in use: 9 bits
-constexpr uint32_t kRadixRounds = 16;     // items per lane per tile
+// items per lane per tile: 16, or 4 for lists too short to give every SM a tile of 16
+constexpr uint32_t kRadixRounds = 16, kRadixRoundsSmall = 4;
 constexpr uint32_t kRadixTile = kRadixThreads * kRadixRounds;
 constexpr uint32_t kMaxPasses = 4;
+static_assert(kRadixThreads >= kRadixBuckets, "one thread per digit in the base scan");
 constexpr unsigned long long kBadKey = 0xffffffffull;   // sorts after every node id
 
 // Look-back status word of (tile, digit): bits 63-62 kind (1 = the tile's own
@@ -126,6 +120,8 @@ __global__ void __launch_bounds__(kRadixThreads) radix_hist_all_kernel(const Id 
                                                                        uint64_t n, uint32_t passes,
                                                                        unsigned long long *items,
                                                                        unsigned long long *hist,
+                                                                       unsigned long long *base,
+                                                                       unsigned long long *done,
                                                                        uint32_t *err)
 {
     constexpr uint32_t NB = 1u << DB, MASK = NB - 1;
@@ -156,21 +152,32 @@ __global__ void __launch_bounds__(kRadixThreads) radix_hist_all_kernel(const Id 
     __syncthreads();
     for (uint32_t b = threadIdx.x; b < passes * NB; b += kRadixThreads)
         if (cnt[b]) atomicAdd(hist + b, (unsigned long long)cnt[b]);
-}
-
-// Exclusive prefix of each pass's digit counts: base[q*NB + b] = items whose
-// pass-q digit is below b.  One block, one thread per pass.
-template <uint32_t DB>
-__global__ void radix_base_kernel(const unsigned long long *hist, uint32_t passes,
-                                  unsigned long long *base)
-{
-    constexpr uint32_t NB = 1u << DB;
-    const uint32_t q = threadIdx.x;
-    if (q >= passes) return;
-    unsigned long long acc = 0;
-    for (uint32_t b = 0; b < NB; ++b) {
-        base[q * NB + b] = acc;
-        acc += hist[q * NB + b];
+    // the last block to come here turns the counts into each pass's digit bases:
+    // base[q*NB + b] = items whose pass-q digit is below b (a kernel of its own,
+    // one thread per pass, took 20-47 us)
+    __shared__ bool last;
+    __shared__ unsigned long long wsum[kRadixWarps];
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(done, 1ull) + 1 == gridDim.x;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    for (uint32_t q = 0; q < passes; ++q) {
+        const unsigned long long c = threadIdx.x < NB ? __ldcg(hist + q * NB + threadIdx.x) : 0ull;
+        unsigned long long x = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const unsigned long long y = __shfl_up_sync(kFull, x, o);
+            if (lane >= (uint32_t)o) x += y;
+        }
+        if (lane == 31) wsum[warp] = x;
+        __syncthreads();
+        unsigned long long before = 0;
+        for (uint32_t w = 0; w < warp; ++w) before += wsum[w];
+        if (threadIdx.x < NB) base[q * NB + threadIdx.x] = before + x - c;
+        __syncthreads();   // wsum is rewritten by the next pass
     }
 }
 
@@ -178,10 +185,10 @@ __global__ void radix_base_kernel(const unsigned long long *hist, uint32_t passe
 // tile is ranked, then the tile in digit order in their place; each digit's
 // global offset less its start within the tile, the warps' bases within the
 // tile, the claimed tile.
-template <uint32_t NB>
+template <uint32_t NB, uint32_t R>
 struct RadixSmem {
     union {
-        unsigned long long stage[kRadixTile];
+        unsigned long long stage[kRadixThreads * R];
         uint2 word[kRadixWarps][NB];   // x: lanes of this round holding the digit, y: count so far
     };
     unsigned long long goff[NB];
@@ -204,7 +211,7 @@ struct RadixSmem {
 // (C2): 8,192-item tiles at two CTAs 224-227 / 75.6 ms; 6,144-item tiles at three
 // CTAs and 40 registers (which spill) 231 / 76.0 ms; 7,168, 9,216 and
 // 10,240-item tiles at two CTAs 231 / 74.2, 238 / 76.8 and 241 / 77.1 ms.
-template <uint32_t DB>
+template <uint32_t DB, uint32_t R>
 __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(
     const unsigned long long *src, unsigned long long *dst, uint64_t n_items, uint32_t shift,
     const unsigned long long *digit_base, unsigned long long *status, uint32_t epoch,
@@ -215,7 +222,7 @@ __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(
     constexpr uint32_t DPT = NB > kRadixThreads ? NB / kRadixThreads : 1;
     static_assert(NB <= kRadixBuckets && DPT * kRadixThreads >= NB, "digit width");
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    RadixSmem<NB> &S = *reinterpret_cast<RadixSmem<NB> *>(smem_raw);
+    RadixSmem<NB, R> &S = *reinterpret_cast<RadixSmem<NB, R> *>(smem_raw);
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t lt = lanemask_lt();
     const bool owner = tid * DPT < NB;
@@ -223,32 +230,32 @@ __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(
     for (uint32_t b = lane; b < NB; b += 32) S.word[warp][b] = make_uint2(0u, 0u);
     __syncthreads();
     const uint64_t t = S.tile;
-    const uint64_t tb = t * kRadixTile;
-    const uint32_t tcount = (uint32_t)min((uint64_t)kRadixTile, n_items - tb);
-    const uint32_t wo = warp * (kRadixRounds * 32);
+    const uint64_t tb = t * (kRadixThreads * R);
+    const uint32_t tcount = (uint32_t)min((uint64_t)(kRadixThreads * R), n_items - tb);
+    const uint32_t wo = warp * (R * 32);
 
     // 1. the digits of the tile's items (the keys, the items' high words), all
     // loads in flight together; the items themselves are read again for the
     // staging, from L2
-    uint32_t dgp[kRadixRounds / 2];   // two digits per register
+    uint32_t dgp[R / 2];   // two digits per register
     {
         const uint32_t *key = reinterpret_cast<const uint32_t *>(src + tb) + 1;
-        uint32_t kv[kRadixRounds];
+        uint32_t kv[R];
 #pragma unroll
-        for (uint32_t r = 0; r < kRadixRounds; ++r) {
+        for (uint32_t r = 0; r < R; ++r) {
             const uint32_t k = wo + r * 32 + lane;
             kv[r] = k < tcount ? key[2 * k] : 0u;
         }
 #pragma unroll
-        for (uint32_t r = 0; r < kRadixRounds; r += 2)
+        for (uint32_t r = 0; r < R; r += 2)
             dgp[r / 2] = ((kv[r] >> shift) & MASK) | (((kv[r + 1] >> shift) & MASK) << 16);
     }
     // stable ranks within the warp's items (in order, 32 per round); two ranks
     // per register
-    uint32_t rk[kRadixRounds / 2];
+    uint32_t rk[R / 2];
     uint2 *const word = S.word[warp];
 #pragma unroll
-    for (uint32_t r = 0; r < kRadixRounds; ++r) {
+    for (uint32_t r = 0; r < R; ++r) {
         const bool valid = wo + r * 32 + lane < tcount;
         const uint32_t dg = (dgp[r / 2] >> ((r & 1) * 16)) & 0xffffu;
         if (valid) atomicOr(&word[dg].x, 1u << lane);
@@ -382,15 +389,15 @@ __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(
     // 5. the tile's items (read a second time) into the stage in digit order;
     // the words under the stage were last read before the barrier above
 #pragma unroll
-    for (uint32_t h = 0; h < kRadixRounds; h += kRadixRounds / 2) {
-        unsigned long long its[kRadixRounds / 2];
+    for (uint32_t h = 0; h < R; h += R / 2) {
+        unsigned long long its[R / 2];
 #pragma unroll
-        for (uint32_t q = 0; q < kRadixRounds / 2; ++q) {
+        for (uint32_t q = 0; q < R / 2; ++q) {
             const uint32_t k = wo + (h + q) * 32 + lane;
             its[q] = k < tcount ? src[tb + k] : 0ull;
         }
 #pragma unroll
-        for (uint32_t q = 0; q < kRadixRounds / 2; ++q) {
+        for (uint32_t q = 0; q < R / 2; ++q) {
             const uint32_t r = h + q;
             if (wo + r * 32 + lane < tcount) {
                 const uint32_t dg = (dgp[r / 2] >> ((r & 1) * 16)) & 0xffffu;
@@ -408,23 +415,15 @@ __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(
     }
 }
 
-// Out entries of rows below x: seed rows from their prefix table, then d per row.
-__device__ __forceinline__ uint64_t outprefix(uint64_t x, uint32_t d, uint64_t seed_edges,
-                                              const int64_t *seed_pre)
+// Out entries of rows below x: the seed rows' closed form (CLIQUE row v holds v
+// edges, to 0..v-1; STAR_REF row d holds d, the others none), then d per row.
+// x <= n < 2^32: one 32-bit product.
+__device__ __forceinline__ uint64_t outprefix(uint64_t x64, uint32_t d, uint64_t seed_edges,
+                                              uint32_t seed_mode)
 {
-    return x <= (uint64_t)d + 1 ? (uint64_t)seed_pre[x] : seed_edges + (x - d - 1) * d;
-}
-
-// seed_pre[x] = out entries of seed rows below x, x = 0..d+1.
-__global__ void seed_prefix_kernel(const uint32_t *seed_out, uint32_t d, int64_t *seed_pre)
-{
-    if (threadIdx.x == 0) {
-        int64_t acc = 0;
-        for (uint32_t x = 0; x <= d + 1; ++x) {
-            seed_pre[x] = acc;
-            if (x <= d) acc += seed_out[x];
-        }
-    }
+    const uint32_t x = (uint32_t)x64;
+    if (x > d) return seed_edges + (uint64_t)(x - d - 1) * d;
+    return seed_mode == PA_SEED_CLIQUE ? (uint64_t)((x * x - x) / 2) : 0ull;
 }
 
 // One pass over the sorted items (the path of d > 32): rowptr[x] = outprefix(x)
@@ -436,7 +435,7 @@ __global__ void seed_prefix_kernel(const uint32_t *seed_out, uint32_t d, int64_t
 // items of one step are a grid stride apart, their loads issued together.
 template <typename Id>
 __global__ void in_sorted_kernel(const unsigned long long *items, uint64_t n_items, uint64_t n,
-                                 uint32_t d, uint64_t seed_edges, const int64_t *seed_pre, Id *col,
+                                 uint32_t d, uint64_t seed_edges, uint32_t seed_mode, Id *col,
                                  uint64_t col_len, int64_t *rowptr)
 {
     constexpr uint32_t U = 4;
@@ -457,9 +456,9 @@ __global__ void in_sorted_kernel(const unsigned long long *items, uint64_t n_ite
             const uint64_t v = i < n_items ? min((uint64_t)(it[q] >> 32), n) : n;
             const uint64_t lo = i > 0 ? min((uint64_t)(pv[q] >> 32), n) + 1 : 0;
             for (uint64_t x = lo; x <= v && x <= n; ++x)
-                rowptr[x] = (int64_t)(outprefix(x, d, seed_edges, seed_pre) + i);
+                rowptr[x] = (int64_t)(outprefix(x, d, seed_edges, seed_mode) + i);
             if (i < n_items && v < n) {
-                const uint64_t pos = outprefix(v + 1, d, seed_edges, seed_pre) + i;
+                const uint64_t pos = outprefix(v + 1, d, seed_edges, seed_mode) + i;
                 if (pos < col_len) col[pos] = (Id)(it[q] & 0xffffffffull);
             }
         }
@@ -468,50 +467,76 @@ __global__ void in_sorted_kernel(const unsigned long long *items, uint64_t n_ite
 
 // rowptr alone (the row writer's input): rowptr[x] = outprefix(x) + the first
 // position k in [0, n_items] whose key is >= x (key(n_items) = n; keys >= n,
-// only after an input error, count as n).  A warp takes 32 * U consecutive
-// positions; for each 32 of them it writes rows (key(k0 - 1), key(k0 + 31)]
-// one per lane, each from the first lane whose key reaches it (a five-step
-// search over the lanes' keys), so a run of rows without in-edges costs one
-// coalesced store per row instead of a loop in one lane.
+// only after an input error, count as n).  A warp takes `span` (32 .. 256, a power
+// of two) consecutive positions and writes rows (key(k0 - 1), key(k0 + span - 1)],
+// one per lane, each from a binary search over the positions' keys, so a run of
+// rows without in-edges costs one coalesced store per row.  Issue-bound, so the
+// search depends on how many rows there are: up to kFewRows, over the whole span
+// in shared memory (one or two steps of 32 rows); more, by shuffles within the 32
+// positions that hold them (five steps instead of eight, no bank conflicts).
+// n = 2.5 * 10^7, d = 16: 1.25 ms by shuffles alone, now 0.75; n = 2^27, d = 4, p = 0.1,
+// CSR: 20.3 ms by shuffles alone, 22.5 in shared memory alone, now 20.4.
+constexpr uint32_t kFewRows = 64;
+constexpr uint32_t kRowSpan = 256;
+
 __global__ void __launch_bounds__(256) rowptr_kernel(const unsigned long long *items, uint64_t n_items,
                                                      uint64_t n, uint32_t d, uint64_t seed_edges,
-                                                     const int64_t *seed_pre, int64_t *rowptr)
+                                                     uint32_t seed_mode, uint32_t span,
+                                                     int64_t *rowptr)
 {
-    constexpr uint32_t U = 8;
+    __shared__ uint32_t s_key[256 / 32][kRowSpan];
     const uint32_t lane = threadIdx.x & 31u;
+    uint32_t *key = s_key[threadIdx.x >> 5];
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     const uint64_t w0 = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const uint64_t positions = n_items + 1;
-    // keys, rows and the search in 32 bits (n < 2^32); rows beyond key(k) are
-    // never written by the lane of k
+    // keys, rows and the search in 32 bits (n < 2^32)
     const uint32_t n32 = (uint32_t)n;
-    for (uint64_t c0 = w0 * 32 * U; c0 < positions; c0 += warps * 32 * U) {
-        uint32_t key[U];
-#pragma unroll
-        for (uint32_t q = 0; q < U; ++q) {
-            const uint64_t k = c0 + q * 32 + lane;
-            key[q] = k < n_items ? (uint32_t)min(items[k] >> 32, (unsigned long long)n) : n32;
-        }
+    for (uint64_t c0 = w0 * span; c0 < positions; c0 += warps * span) {
         // the first row not yet written: rows up to key(c0 - 1) belong to the
         // warp holding position c0 - 1
         uint64_t nxt = c0 == 0 ? 0 : min(items[c0 - 1] >> 32, (unsigned long long)n) + 1;
+        uint32_t v[kRowSpan / 32];
 #pragma unroll
-        for (uint32_t q = 0; q < U; ++q) {
-            const uint64_t kb = c0 + q * 32;
-            if (kb >= positions) break;   // warp-uniform
-            const uint32_t v = key[q];
-            const uint32_t last = __shfl_sync(kFull, v, 31);
+        for (uint32_t q = 0; q < kRowSpan / 32; ++q) {
+            const uint64_t k = c0 + q * 32 + lane;
+            v[q] = n32;
+            if (q * 32 < span && k < n_items)
+                v[q] = (uint32_t)min(items[k] >> 32, (unsigned long long)n);
+        }
+        __syncwarp();
+#pragma unroll
+        for (uint32_t q = 0; q < kRowSpan / 32; ++q)
+            if (q * 32 < span) key[q * 32 + lane] = v[q];
+        __syncwarp();
+        const uint32_t last = key[span - 1];
+        if (last <= nxt + kFewRows) {
             for (uint64_t x0 = nxt; x0 <= last; x0 += 32) {
                 const uint64_t x = x0 + lane;
-                const uint32_t xs = (uint32_t)min(x, (uint64_t)last);
+                if (x <= last) {
+                    uint32_t lo = 0;   // positions of the span whose key is below x
+                    for (uint32_t step = span / 2; step > 0; step >>= 1)
+                        if (key[lo + step - 1] < (uint32_t)x) lo += step;
+                    rowptr[x] = (int64_t)(outprefix(x, d, seed_edges, seed_mode) + c0 + lo);
+                }
+            }
+            continue;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kRowSpan / 32; ++q) {
+            if (q * 32 >= span) break;   // warp-uniform
+            const uint32_t last_q = __shfl_sync(kFull, v[q], 31);
+            for (uint64_t x0 = nxt; x0 <= last_q; x0 += 32) {
+                const uint64_t x = x0 + lane;
+                const uint32_t xs = (uint32_t)min(x, (uint64_t)last_q);
                 uint32_t lo = 0;   // lanes whose key is below x
 #pragma unroll
                 for (uint32_t step = 16; step > 0; step >>= 1)
-                    if (__shfl_sync(kFull, v, lo + step - 1) < xs) lo += step;
-                if (x <= last)
-                    rowptr[x] = (int64_t)(outprefix(x, d, seed_edges, seed_pre) + kb + lo);
+                    if (__shfl_sync(kFull, v[q], lo + step - 1) < xs) lo += step;
+                if (x <= last_q)
+                    rowptr[x] = (int64_t)(outprefix(x, d, seed_edges, seed_mode) + c0 + q * 32 + lo);
             }
-            if ((uint64_t)last + 1 > nxt) nxt = (uint64_t)last + 1;
+            if ((uint64_t)last_q + 1 > nxt) nxt = (uint64_t)last_q + 1;
         }
     }
 }
@@ -524,25 +549,43 @@ __global__ void __launch_bounds__(256) rowptr_kernel(const unsigned long long *i
 // every row boundary, which DRAM then reads and writes back twice.)
 //
 // Row x's in part is sorted items [lb(x), lb(x+1)), lb(x) = rowptr[x] -
-// outprefix(x); entry k of it (item index) goes to col[outprefix(x+1) + k].
-// A row whose in part is longer than kHeavyIn items is listed here and its in
-// part copied in pieces of kPiece items spread over all warps (heavy_scan_kernel,
-// heavy_in_kernel), so that hub rows -- up to every item at p = 0 -- hold no
-// single warp or block.
+// outprefix(x); entry k of it (item index) goes to col[outprefix(x+1) + k], so the
+// in parts of a chunk are one range of items, and any warp can copy any piece of
+// it.  A chunk whose range is longer than heavy_limit -- it holds hub rows, up
+// to every item at p = 0 -- is listed here and copied in pieces of kPiece items
+// spread over all warps (heavy_in_kernel), so that it holds up no single warp.
+// (Listing rows of more than 512 in-edges instead left the 32 first rows of a
+// graph of 2 * 10^4 nodes, d = 6, to one warp: 52 us of the row writer, now 9-12.)
 // ---------------------------------------------------------------------------
 constexpr uint32_t kRowsChunk = 32;        // rows per warp step: one per lane
-constexpr uint64_t kHeavyIn = 512;         // longest in part a row warp copies
-constexpr uint32_t kPiece = 512;           // items per piece of a longer one
+constexpr uint64_t kHeavyMin = 1024;       // least heavy_limit
+constexpr uint32_t kPiece = 512;           // items per piece of a listed chunk
+// The list's counter: listed chunks in the high bits, their pieces below (one
+// atomic gives a chunk its place and its first piece, both in the same order).
+constexpr uint32_t kHeavyShift = 36;
+constexpr unsigned long long kPieceMask = (1ull << kHeavyShift) - 1;
+
+// In items of a chunk (32 d on average) a row warp copies by itself.  Rows and in
+// parts written together share their sectors, so a large graph, where a warp has
+// many chunks, lists only what is more than a warp's even share of all items
+// (n = 2.5 * 10^7, d = 16, a limit of 1,024 instead of 16,384: the pieces take
+// 0.77 ms of 3.51 instead of 0.07 of 3.40).
+__device__ __forceinline__ uint64_t heavy_limit(uint64_t n_items, uint64_t warps, uint32_t d)
+{
+    return min(16384ull, max(max((unsigned long long)kHeavyMin, 64ull * d),
+                             (unsigned long long)(n_items / warps)));
+}
 
 __device__ __forceinline__ uint64_t clamp_items(int64_t v, uint64_t n_items)
 {
     return v < 0 ? 0ull : ((uint64_t)v > n_items ? n_items : (uint64_t)v);
 }
 
-// Out degree of row x: seed rows from the prefix table, d for the others.
-__device__ __forceinline__ uint32_t outdeg(uint64_t x, uint32_t d, const int64_t *seed_pre)
+// Out degree of row x.
+__device__ __forceinline__ uint32_t outdeg(uint64_t x, uint32_t d, uint32_t seed_mode)
 {
-    return x <= (uint64_t)d ? (uint32_t)(seed_pre[x + 1] - seed_pre[x]) : d;
+    if (x >= d) return d;
+    return seed_mode == PA_SEED_CLIQUE ? (uint32_t)x : 0u;
 }
 
 // Copy sorted items [a, b) -- the in parts of some of a row warp's rows -- into
@@ -550,7 +593,7 @@ __device__ __forceinline__ uint32_t outdeg(uint64_t x, uint32_t d, const int64_t
 template <typename Id>
 __device__ __forceinline__ void copy_in_items(const unsigned long long *items, uint64_t a, uint64_t b,
                                               uint32_t lane, uint64_t n, uint32_t d,
-                                              uint64_t seed_edges, const int64_t *seed_pre, Id *col,
+                                              uint64_t seed_edges, uint32_t seed_mode, Id *col,
                                               uint64_t col_len)
 {
     constexpr uint32_t U = 4;
@@ -566,7 +609,7 @@ __device__ __forceinline__ void copy_in_items(const unsigned long long *items, u
             const uint64_t k = k0 + q * 32 + lane;
             const uint64_t v = it[q] >> 32;
             if (k < b && v < n) {
-                const uint64_t pos = outprefix(v + 1, d, seed_edges, seed_pre) + k;
+                const uint64_t pos = outprefix(v + 1, d, seed_edges, seed_mode) + k;
                 if (pos < col_len) col[pos] = (Id)(it[q] & 0xffffffffull);
             }
         }
@@ -577,8 +620,9 @@ template <typename Id>
 __global__ void __launch_bounds__(256) rows_kernel(const Id *E, const unsigned long long *items,
                                                    uint64_t n_items, const int64_t *rowptr, Id *col,
                                                    uint64_t n, uint32_t d, uint64_t seed_edges,
-                                                   const int64_t *seed_pre, uint64_t col_len,
-                                                   unsigned long long *heavy, uint64_t heavy_cap,
+                                                   uint32_t seed_mode, uint64_t col_len,
+                                                   unsigned long long *heavy,
+                                                   unsigned long long *pref, uint64_t heavy_cap,
                                                    unsigned long long *ctr)
 {
     const uint32_t lane = threadIdx.x & 31u;
@@ -588,44 +632,46 @@ __global__ void __launch_bounds__(256) rows_kernel(const Id *E, const unsigned l
     const uint32_t g = lane / d, i = lane - g * d;
     const bool used = lane < G * d;
     const uint64_t step = warps * kRowsChunk;
-    // rowptr of each chunk's rows is loaded one chunk ahead
-    int64_t rp_next = 0, rp1_next = 0;
-    if (w0 * kRowsChunk + lane < n) {
-        rp_next = rowptr[w0 * kRowsChunk + lane];
-        rp1_next = rowptr[w0 * kRowsChunk + lane + 1];
+    const uint64_t limit = heavy_limit(n_items, warps, d);
+    // rowptr of each chunk's rows, and of the row after it, is loaded one chunk
+    // ahead
+    int64_t rp_next = 0, re_next = 0;
+    if (w0 * kRowsChunk < n) {
+        rp_next = rowptr[min(w0 * kRowsChunk + lane, n)];
+        re_next = rowptr[min((w0 + 1) * kRowsChunk, n)];
     }
     for (uint64_t x0 = w0 * kRowsChunk; x0 < n; x0 += step) {
-        // lane j: row x0 + j, its rowptr and its in part's item range
-        const uint64_t x = x0 + lane;
-        const bool row_ok = x < n;
-        const int64_t rp = row_ok ? rp_next : 0, rp1 = row_ok ? rp1_next : 0;
-        if (x + step < n) {
-            rp_next = rowptr[x + step];
-            rp1_next = rowptr[x + step + 1];
+        // lane j: row x0 + j and its rowptr
+        const int64_t rp = rp_next, re = re_next;
+        if (x0 + step < n) {
+            rp_next = rowptr[min(x0 + step + lane, n)];
+            re_next = rowptr[min(x0 + step + kRowsChunk, n)];
         }
-        uint64_t lb = n_items, lb1 = n_items;
-        if (row_ok) {
-            lb = clamp_items(rp - (int64_t)outprefix(x, d, seed_edges, seed_pre), n_items);
-            lb1 = clamp_items(rp1 - (int64_t)outprefix(x + 1, d, seed_edges, seed_pre), n_items);
-            if (lb1 < lb) lb1 = lb;
+        // the chunk's in parts: items [a, end)
+        uint64_t a = clamp_items(
+            __shfl_sync(kFull, rp, 0) - (int64_t)outprefix(x0, d, seed_edges, seed_mode), n_items);
+        uint64_t end = clamp_items(
+            re - (int64_t)outprefix(min(x0 + kRowsChunk, n), d, seed_edges, seed_mode), n_items);
+        if (end > a + limit) {
+            if (lane == 0) {
+                // listed in any order: every entry's place is fixed by its index
+                const unsigned long long old =
+                    atomicAdd(ctr, (1ull << kHeavyShift) | ((end - a + kPiece - 1) / kPiece));
+                const uint64_t slot = old >> kHeavyShift;
+                if (slot < heavy_cap) {
+                    heavy[slot] = x0;
+                    pref[slot] = old & kPieceMask;
+                }
+            }
+            end = a;   // nothing to copy here
         }
-        const bool heavy_row = row_ok && lb1 - lb > kHeavyIn;
-        if (heavy_row) {
-            // listed in any order: every entry's place is fixed by its index
-            const unsigned long long slot = atomicAdd(ctr, 1ull);
-            if (slot < heavy_cap) heavy[slot] = x;
-        }
-        uint32_t hv = __ballot_sync(kFull, heavy_row);
-        uint64_t a = __shfl_sync(kFull, lb, 0);
-        const uint64_t end = __shfl_sync(kFull, lb1, 31);
-        // without hub rows the chunk's in parts are items [a, end): their first
-        // kPre * 32 loads go out now, beside the out parts' loads below
+        // the first kPre * 32 loads go out now, beside the out parts' loads below
         constexpr uint32_t kPre = 4;
         unsigned long long pre[kPre];
 #pragma unroll
         for (uint32_t q = 0; q < kPre; ++q) {
             const uint64_t k = a + q * 32 + lane;
-            pre[q] = hv == 0 && k < end ? items[k] : ~0ull;
+            pre[q] = k < end ? items[k] : ~0ull;
         }
 
         // (a) out parts, G rows per pass, each row's d targets ranked in
@@ -648,7 +694,7 @@ __global__ void __launch_bounds__(256) rows_kernel(const Id *E, const unsigned l
                 if (act && row > d) {
                     t[q] = (uint32_t)E[2 * (seed_edges + (row - d - 1) * d + i) + 1];
                     have[q] = true;
-                } else if (act && i < outdeg(row, d, seed_pre)) {
+                } else if (act && i < outdeg(row, d, seed_mode)) {
                     t[q] = i;
                     have[q] = true;
                 }
@@ -674,102 +720,24 @@ __global__ void __launch_bounds__(256) rows_kernel(const Id *E, const unsigned l
             }
         }
 
-        // (b) in parts of the chunk's rows, the heavy rows' ranges skipped
-        if (hv == 0) {
+        // (b) in parts of the chunk's rows
 #pragma unroll
-            for (uint32_t q = 0; q < kPre; ++q) {
-                const uint64_t k = a + q * 32 + lane;
-                const uint64_t v = pre[q] >> 32;
-                if (k < end && v < n) {
-                    const uint64_t pos = outprefix(v + 1, d, seed_edges, seed_pre) + k;
-                    if (pos < col_len) col[pos] = (Id)(pre[q] & 0xffffffffull);
-                }
+        for (uint32_t q = 0; q < kPre; ++q) {
+            const uint64_t k = a + q * 32 + lane;
+            const uint64_t v = pre[q] >> 32;
+            if (k < end && v < n) {
+                const uint64_t pos = outprefix(v + 1, d, seed_edges, seed_mode) + k;
+                if (pos < col_len) col[pos] = (Id)(pre[q] & 0xffffffffull);
             }
-            a = min(a + kPre * 32, end);
         }
-        while (true) {
-            uint64_t b = end, next = end;
-            if (hv) {
-                const uint32_t h = __ffs(hv) - 1;
-                b = __shfl_sync(kFull, lb, h);
-                next = __shfl_sync(kFull, lb1, h);
-                hv &= hv - 1;
-            }
-            if (b > a) copy_in_items(items, a, b, lane, n, d, seed_edges, seed_pre, col, col_len);
-            if (b == end && next == end) break;
-            a = next;
-        }
+        if (a + kPre * 32 < end)
+            copy_in_items(items, a + kPre * 32, end, lane, n, d, seed_edges, seed_mode, col, col_len);
     }
 }
 
-// Row x's in part: sorted items [lb, lb1), entry k at col[base + k].
-struct InPart {
-    uint64_t lb, lb1, base;
-};
-
-__device__ __forceinline__ InPart in_part(uint64_t x, const int64_t *rowptr, uint64_t n_items,
-                                          uint32_t d, uint64_t seed_edges, const int64_t *seed_pre)
-{
-    InPart r;
-    r.base = outprefix(x + 1, d, seed_edges, seed_pre);
-    r.lb = clamp_items(rowptr[x] - (int64_t)outprefix(x, d, seed_edges, seed_pre), n_items);
-    r.lb1 = clamp_items(rowptr[x + 1] - (int64_t)r.base, n_items);
-    if (r.lb1 < r.lb) r.lb1 = r.lb;
-    return r;
-}
-
-// The first piece of every listed row: pref[h] = pieces of rows 0..h-1 of the
-// list, pref[K] = all pieces (one block; the list holds at most one entry per
-// kHeavyIn items).
-__global__ void __launch_bounds__(1024) heavy_scan_kernel(const unsigned long long *heavy,
-                                                          uint64_t heavy_cap,
-                                                          const unsigned long long *ctr,
-                                                          const int64_t *rowptr, uint64_t n,
-                                                          uint32_t d, uint64_t seed_edges,
-                                                          const int64_t *seed_pre,
-                                                          uint64_t n_items,
-                                                          unsigned long long *pref)
-{
-    __shared__ unsigned long long wsum[32];
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint64_t K = min((uint64_t)ctr[0], heavy_cap);
-    unsigned long long carry = 0;
-    for (uint64_t h0 = 0; h0 < K; h0 += 1024) {
-        const uint64_t h = h0 + threadIdx.x;
-        unsigned long long pc = 0;
-        if (h < K && heavy[h] < n) {
-            const InPart r = in_part(heavy[h], rowptr, n_items, d, seed_edges, seed_pre);
-            pc = (r.lb1 - r.lb + kPiece - 1) / kPiece;
-        }
-        unsigned long long x = pc;   // inclusive scan over the block
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const unsigned long long y = __shfl_up_sync(kFull, x, o);
-            if (lane >= (uint32_t)o) x += y;
-        }
-        if (lane == 31) wsum[warp] = x;
-        __syncthreads();
-        if (warp == 0) {
-            unsigned long long w = wsum[lane];
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const unsigned long long y = __shfl_up_sync(kFull, w, o);
-                if (lane >= (uint32_t)o) w += y;
-            }
-            wsum[lane] = w;
-        }
-        __syncthreads();
-        const unsigned long long before = warp > 0 ? wsum[warp - 1] : 0ull;
-        if (h < K) pref[h] = carry + before + x - pc;
-        carry += wsum[31];
-        __syncthreads();   // wsum is rewritten by the next chunk
-    }
-    if (threadIdx.x == 0) pref[K] = carry;
-}
-
-// In parts of the listed rows, in pieces of kPiece items: a warp takes runs of
-// kPieceRun consecutive pieces (over all listed rows, in list order), finds the
-// row of its first piece by binary search over pref and copies each piece with
+// In parts of the listed chunks, in pieces of kPiece items: a warp takes runs of
+// consecutive pieces, kPieceRun at most and one where there are few (over all
+// listed chunks, in list order), finds the chunk of its first piece by binary search over pref and copies each piece with
 // all 32 lanes (kPiece / 32 items each, loads issued together).
 constexpr uint32_t kPieceRun = 16;
 
@@ -777,50 +745,60 @@ template <typename Id>
 __global__ void __launch_bounds__(256) heavy_in_kernel(const unsigned long long *items,
                                                        uint64_t n_items, const int64_t *rowptr,
                                                        Id *col, uint64_t n, uint32_t d,
-                                                       uint64_t seed_edges, const int64_t *seed_pre,
+                                                       uint64_t seed_edges, uint32_t seed_mode,
                                                        uint64_t col_len,
                                                        const unsigned long long *heavy,
+                                                       const unsigned long long *pref,
                                                        uint64_t heavy_cap,
-                                                       const unsigned long long *ctr,
-                                                       const unsigned long long *pref)
+                                                       const unsigned long long *ctr)
 {
     constexpr uint32_t PL = kPiece / 32;   // items per lane per piece
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     const uint64_t w0 = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const uint64_t K = min((uint64_t)ctr[0], heavy_cap);
+    const uint64_t K = min((uint64_t)(ctr[0] >> kHeavyShift), heavy_cap);
     if (K == 0) return;
-    const uint64_t T = pref[K];
-    for (uint64_t t0 = w0 * kPieceRun; t0 < T; t0 += warps * kPieceRun) {
-        // the last h with pref[h] <= t0 (pref[0] = 0, pref is non-decreasing)
-        uint64_t lo = 0, hi = K;
-        while (hi - lo > 1) {
-            const uint64_t mid = lo + (hi - lo) / 2;
-            if (pref[mid] <= t0) lo = mid;
+    const uint64_t T = ctr[0] & kPieceMask;
+    const uint64_t run = min((uint64_t)kPieceRun, max((uint64_t)1, T / warps));
+    for (uint64_t t0 = w0 * run; t0 < T; t0 += warps * run) {
+        // the last h with pref[h] <= t0 (pref[0] = 0, pref is increasing)
+        uint64_t h = 0, hi = K;
+        while (hi - h > 1) {
+            const uint64_t mid = h + (hi - h) / 2;
+            if (pref[mid] <= t0) h = mid;
             else hi = mid;
         }
-        uint64_t h = lo, next = pref[h + 1];
-        InPart r{0, 0, 0};
-        if (heavy[h] < n) r = in_part(heavy[h], rowptr, n_items, d, seed_edges, seed_pre);
-        const uint64_t t1 = min(t0 + kPieceRun, T);
+        uint64_t next = 0, first = 0, a = 0, end = 0;   // the chunk's pieces and items
+        bool open = false;
+        const uint64_t t1 = min(t0 + run, T);
         for (uint64_t t = t0; t < t1; ++t) {
-            while (t >= next && h + 1 < K) {   // rows of one piece or more: a few steps
-                ++h;
-                next = pref[h + 1];
-                r = heavy[h] < n ? in_part(heavy[h], rowptr, n_items, d, seed_edges, seed_pre)
-                                 : InPart{0, 0, 0};
+            if (open && t >= next) {
+                ++h;   // every chunk has a piece at least
+                open = false;
             }
-            const uint64_t k0 = r.lb + (t - pref[h]) * kPiece;
+            if (!open) {
+                const uint64_t x0 = min((uint64_t)heavy[h], n), x1 = min(x0 + kRowsChunk, n);
+                first = pref[h];
+                next = h + 1 < K ? pref[h + 1] : T;
+                a = clamp_items(rowptr[x0] - (int64_t)outprefix(x0, d, seed_edges, seed_mode), n_items);
+                end = clamp_items(rowptr[x1] - (int64_t)outprefix(x1, d, seed_edges, seed_mode),
+                                  n_items);
+                open = true;
+            }
+            const uint64_t k0 = a + (t - first) * kPiece;
             unsigned long long it[PL];
 #pragma unroll
             for (uint32_t q = 0; q < PL; ++q) {
                 const uint64_t k = k0 + q * 32 + lane;
-                it[q] = k < r.lb1 ? items[k] : 0ull;
+                it[q] = k < end ? items[k] : ~0ull;
             }
 #pragma unroll
             for (uint32_t q = 0; q < PL; ++q) {
-                const uint64_t k = k0 + q * 32 + lane, pos = r.base + k;
-                if (k < r.lb1 && pos < col_len) col[pos] = (Id)(it[q] & 0xffffffffull);
+                const uint64_t k = k0 + q * 32 + lane, v = it[q] >> 32;
+                if (k < end && v < n) {
+                    const uint64_t pos = outprefix(v + 1, d, seed_edges, seed_mode) + k;
+                    if (pos < col_len) col[pos] = (Id)(it[q] & 0xffffffffull);
+                }
             }
         }
     }
@@ -837,10 +815,11 @@ int grid_for(uint64_t items, uint32_t threads, uint32_t per_sm = 8)
 }
 
 struct CsrLayout {
-    uint64_t items_off, status_off, hist_off, base_off, ctr_off, err_off, seed_out_off,
-        seed_pre_off, heavy_off, pref_off, total;
+    // ctr: one tile counter per pass, the listed chunks' counter, the histogram
+    // blocks done; then the error word and the digit counts, cleared together
+    uint64_t items_off, status_off, ctr_off, err_off, hist_off, base_off, heavy_off, pref_off, total;
     uint64_t r_tiles;               // radix tiles
-    uint64_t heavy_cap;             // rows with in parts above kHeavyIn items
+    uint64_t heavy_cap;             // room in the list of chunks
     uint32_t db, passes;            // digit bits and passes of the sort
     uint64_t status_bytes;
     bool status_in_col;             // status words in the column buffer's second half
@@ -886,39 +865,37 @@ CsrLayout csr_layout(uint64_t n, uint32_t d, uint64_t n_edges, uint32_t id_bytes
     uint64_t o = 0;
     L.items_off = o;    o += al(8 * std::max<uint64_t>(n_edges, 1));
     L.status_off = o;   o += L.status_in_col ? 0 : al(L.status_bytes);
+    L.ctr_off = o;      o += 256;
+    L.err_off = o;      o += 256;
     L.hist_off = o;     o += al(8 * kMaxPasses * kRadixBuckets);
     L.base_off = o;     o += al(8 * kMaxPasses * kRadixBuckets);
-    L.ctr_off = o;      o += 256;   // one tile counter per pass, then the hub rows'
-    L.err_off = o;      o += 256;
-    L.seed_out_off = o; o += al(4 * (d + 1));
-    L.seed_pre_off = o; o += al(8 * (d + 2));
-    // more than cap rows cannot each hold more than kHeavyIn of the n_edges items
-    L.heavy_cap = n_edges / (kHeavyIn + 1) + 1;
-
+    // more chunks than this cannot each hold more than kHeavyMin of the n_edges items
+    // (half of it could; the size callers have planned with)
+    L.heavy_cap = n_edges / 513 + 1;
     L.heavy_off = o;    o += al(8 * L.heavy_cap);
     L.pref_off = o;     o += al(8 * (L.heavy_cap + 1));
+    o += al(4 * (d + 1)) + al(8 * (d + 2));   // unused: the size callers have planned with
     L.total = o;
     return L;
 }
 
 // Every pass of the sort: the histogram of all passes' digits, their bases,
 // then one kernel per pass.  The last pass always lands in A.
-template <typename Id, uint32_t DB>
+template <typename Id, uint32_t DB, uint32_t R>
 int radix_sort(const Id *E, uint64_t m, uint64_t n, uint32_t passes, unsigned long long *A,
                unsigned long long *B, unsigned long long *status, unsigned char *scratch,
                const CsrLayout &L, uint32_t *err, cudaStream_t s)
 {
     constexpr uint32_t NB = 1u << DB;
+    const uint64_t r_tiles = (m + kRadixThreads * R - 1) / (kRadixThreads * R);
     unsigned long long *hist = (unsigned long long *)(scratch + L.hist_off);
     unsigned long long *base = (unsigned long long *)(scratch + L.base_off);
     unsigned long long *ctr = (unsigned long long *)(scratch + L.ctr_off);
-    const size_t smem = sizeof(RadixSmem<NB>);
-    cudaError_t e = cudaFuncSetAttribute(radix_pass_kernel<DB>,
+    const size_t smem = sizeof(RadixSmem<NB, R>);
+    cudaError_t e = cudaFuncSetAttribute(radix_pass_kernel<DB, R>,
                                          cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     // status words of an earlier call must not read as this call's
-    if (e == cudaSuccess) e = cudaMemsetAsync(status, 0, 8 * (uint64_t)NB * L.r_tiles, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(hist, 0, 8 * kMaxPasses * kRadixBuckets, s);
-    if (e == cudaSuccess) e = cudaMemsetAsync(ctr, 0, 8 * kMaxPasses, s);
+    if (e == cudaSuccess) e = cudaMemsetAsync(status, 0, 8 * (uint64_t)NB * r_tiles, s);
     if (e != cudaSuccess) return set_cuda_error(e);
     // pass q reads what pass q - 1 wrote; the histogram kernel writes the
     // items where pass 0 reads them, so that the last pass lands in A
@@ -927,11 +904,10 @@ int radix_sort(const Id *E, uint64_t m, uint64_t n, uint32_t passes, unsigned lo
     // n = 10^8, d = 16 the kernel took 8.44 ms with two blocks per SM, 5.96 ms
     // with four
     radix_hist_all_kernel<Id, DB><<<grid_for(m / 4 + 1, kRadixThreads, 4), kRadixThreads, 0, s>>>(
-        E, m, n, passes, buf(0), hist, err);
-    radix_base_kernel<DB><<<1, 32, 0, s>>>(hist, passes, base);
-    const unsigned tiles = (unsigned)L.r_tiles;
+        E, m, n, passes, buf(0), hist, base, ctr + kMaxPasses + 1, err);
+    const unsigned tiles = (unsigned)r_tiles;
     for (uint32_t q = 0; q < passes; ++q)
-        radix_pass_kernel<DB><<<tiles, kRadixThreads, smem, s>>>(
+        radix_pass_kernel<DB, R><<<tiles, kRadixThreads, smem, s>>>(
             buf(q), buf(q + 1), m, DB * q, base + q * NB, status, q + 1, ctr + q, 2000000000ull, err);
     e = cudaGetLastError();
     return e == cudaSuccess ? PA_OK : set_cuda_error(e);
@@ -945,26 +921,38 @@ int csr_enqueue_t(const pa_params *prm, const GenPlan &p, const Id *E, int64_t *
 {
     const uint64_t n = prm->n, m = p.n_edges;
     const uint32_t d = prm->d;
-    uint32_t *seed_out = (uint32_t *)(scratch + L.seed_out_off);
-    int64_t *seed_pre = (int64_t *)(scratch + L.seed_pre_off);
     uint32_t *err = (uint32_t *)(scratch + L.err_off);
     unsigned long long *A = (unsigned long long *)(scratch + L.items_off);
     // the column buffer (>= 8 bytes per pair) holds the other ping-pong array
     // while sorting; the last pass always lands in A
     unsigned long long *B = reinterpret_cast<unsigned long long *>(col);
-    cudaError_t e = cudaMemsetAsync(err, 0, 4, s);
+    // the counters, the error word and the digit counts lie back to back
+    cudaError_t e = cudaMemsetAsync(scratch + L.ctr_off, 0, L.base_off - L.ctr_off, s);
     if (e != cudaSuccess) return set_cuda_error(e);
-    seed_out_kernel<<<1, 256, 0, s>>>(d, prm->seed_mode, seed_out);
-    seed_prefix_kernel<<<1, 32, 0, s>>>(seed_out, d, seed_pre);
+    const uint32_t seed_mode = prm->seed_mode;
     unsigned long long *status =
         L.status_in_col ? reinterpret_cast<unsigned long long *>(col) + m
                         : (unsigned long long *)(scratch + L.status_off);
     if (m > 0) {
         int rc = PA_ERR_INVALID;
-        if (L.db == 9)
-            rc = radix_sort<Id, 9>(E, m, n, L.passes, A, B, status, scratch, L, err, s);
-        else
-            rc = radix_sort<Id, 8>(E, m, n, L.passes, A, B, status, scratch, L, err, s);
+        // small tiles where tiles of 8,192 would leave SMs idle (n = 2 * 10^4, d = 6:
+        // 15 of them; a pass 11.5 -> 8.9 us), if their look-back words -- four times as many
+        // -- fit the column buffer's half or the row starts, not written yet
+        constexpr uint64_t kSmallTile = kRadixThreads * kRadixRoundsSmall;
+        const uint64_t small_bytes = (8ull << L.db) * ((m + kSmallTile - 1) / kSmallTile);
+        bool small = m <= 148 * (uint64_t)kRadixTile;
+        if (p.id_bytes == 8 && small_bytes <= 8 * m) {
+            if (small) status = reinterpret_cast<unsigned long long *>(col) + m;
+        } else if (small && small_bytes <= 8 * (n + 1)) {
+            status = reinterpret_cast<unsigned long long *>(rowptr);
+        } else {
+            small = false;
+        }
+        auto sort = small ? (L.db == 9 ? radix_sort<Id, 9, kRadixRoundsSmall>
+                                       : radix_sort<Id, 8, kRadixRoundsSmall>)
+                          : (L.db == 9 ? radix_sort<Id, 9, kRadixRounds>
+                                       : radix_sort<Id, 8, kRadixRounds>);
+        rc = sort(E, m, n, L.passes, A, B, status, scratch, L, err, s);
         if (rc != PA_OK) return rc;
     }
     const uint64_t col_len = 2 * m;
@@ -972,29 +960,28 @@ int csr_enqueue_t(const pa_params *prm, const GenPlan &p, const Id *E, int64_t *
         // in parts and rowptr from the sorted items, the seed rows' out parts,
         // then the generated rows' out parts (ranked in shared memory)
         in_sorted_kernel<Id><<<grid_for(m / 4 + 1, 256), 256, 0, s>>>(
-            A, m, n, d, p.seed_edges, seed_pre, col, col_len, rowptr);
+            A, m, n, d, p.seed_edges, seed_mode, col, col_len, rowptr);
         seed_out_part_kernel<Id><<<grid_for(p.seed_edges, 256), 256, 0, s>>>(E, rowptr, col, n,
                                                                              p.seed_edges, col_len);
         const int rc = gen::csr_out_wide(p.id_bytes, E, rowptr, col, n, d, p.seed_edges, col_len, s);
         if (rc != PA_OK) return rc;
     } else {
-        // rowptr, then whole rows (the hub rows' in parts listed and copied last)
+        // rowptr, then whole rows (the in parts of chunks with hub rows listed and copied last)
         unsigned long long *lists = (unsigned long long *)(scratch + L.ctr_off) + kMaxPasses;
         unsigned long long *heavy = (unsigned long long *)(scratch + L.heavy_off);
         unsigned long long *pref = (unsigned long long *)(scratch + L.pref_off);
-        e = cudaMemsetAsync(lists, 0, 8, s);
-        if (e != cudaSuccess) return set_cuda_error(e);
-        rowptr_kernel<<<grid_for(m / 8 + 1, 256), 256, 0, s>>>(A, m, n, d, p.seed_edges,
-                                                                seed_pre, rowptr);
+        // fewer positions a warp where 256 would leave SMs without work (a warp at
+        // the end of a graph, where few rows have in-edges, writes hundreds)
+        uint32_t span = kRowSpan;
+        while (span > 32 && m < (uint64_t)span * 148 * 64) span /= 2;
+        rowptr_kernel<<<grid_for(m / span + 1, 256 / 32), 256, 0, s>>>(A, m, n, d, p.seed_edges,
+                                                                       seed_mode, span, rowptr);
         const int grid = grid_for(n / kRowsChunk + 1, 256 / 32);
-        rows_kernel<Id><<<grid, 256, 0, s>>>(E, A, m, rowptr, col, n, d, p.seed_edges, seed_pre,
-                                             col_len, heavy, L.heavy_cap, lists);
-        heavy_scan_kernel<<<1, 1024, 0, s>>>(heavy, L.heavy_cap, lists, rowptr, n, d,
-                                              p.seed_edges, seed_pre, m, pref);
-        // one warp per run of kPieceRun pieces; at most m / kPiece + (listed rows) pieces
-        heavy_in_kernel<Id><<<grid_for(m / (kPiece * kPieceRun) + 1, 256 / 32), 256, 0, s>>>(
-            A, m, rowptr, col, n, d, p.seed_edges, seed_pre, col_len, heavy, L.heavy_cap, lists,
-            pref);
+        rows_kernel<Id><<<grid, 256, 0, s>>>(E, A, m, rowptr, col, n, d, p.seed_edges, seed_mode,
+                                             col_len, heavy, pref, L.heavy_cap, lists);
+        // one warp per piece at least; at most m / kPiece + (listed chunks) pieces
+        heavy_in_kernel<Id><<<grid_for(m / kPiece + 1, 256 / 32), 256, 0, s>>>(
+            A, m, rowptr, col, n, d, p.seed_edges, seed_mode, col_len, heavy, pref, L.heavy_cap, lists);
     }
     e = cudaGetLastError();
     return e == cudaSuccess ? PA_OK : set_cuda_error(e);
