@@ -70,8 +70,6 @@ int make_plan(const pa_params *prm, GenPlan *plan)
                                              : kStartNodesAuto;
     p.u_split = p.wide ? prm->n
                        : start_split(prm->n, p.u_first, (uint64_t)kSbTiles * p.tile_nodes, want);
-    const uint64_t st_nodes = (uint64_t)kStartPasses * p.groups;
-    p.start_tiles = p.wide ? 0 : (p.u_split - p.u_first + st_nodes - 1) / st_nodes;
     p.scratch_bytes = p.start_offset + kStartAreaBytes;
     p.claim_tiles = prm->claim_tiles ? prm->claim_tiles : kClaimTilesAuto;
     *plan = p;

@@ -15,23 +15,38 @@ namespace gen {
 constexpr uint32_t kFull = 0xffffffffu;
 constexpr uint32_t kThreads = 256;
 constexpr uint32_t kMinBlocks = 4;   // 32 resident warps per SM: at most 64 registers
-// The start kernel: 40 warps per SM (at most 51 registers; a few bytes spill).
-// More warps put more copy reads in flight: C3 69.4 -> 68.2 ms at p = 0.5.
+// The start kernel's variants: resident blocks of 8 warps per SM, and warp passes
+// per tile.
+//  * kStartMinBlocks: 40 warps (at most 51 registers; a few bytes spill).
+//  * kStartMinBlocksMid: 32 warps, 64 registers, no spills.
+//  * kStartMinBlocksMany: 48 warps.
 constexpr uint32_t kStartMinBlocks = 5;
-// p = 0 (every slot a copy, several retries per node): 48 warps per SM pay off
-// there (C3 270 -> 259 ms) though they cost at p = 0.5 (68.1 -> 71.7 ms).
-constexpr uint32_t kStartMinBlocksCopy = 6;
-// A single graph with a small start region is bound by its dependency chains'
-// latency, which the spills of the wider variants lengthen: four blocks, 64
-// registers, no spills.
-constexpr uint32_t kStartMinBlocksSmall = 4;
-constexpr uint64_t kStartLargeNodes = 1ull << 24;
+constexpr uint32_t kStartMinBlocksMid = 4;
+constexpr uint32_t kStartMinBlocksMany = 6;
+struct StartVariant {
+    uint32_t min_blocks, passes;
+};
 
-// The start-kernel variant for one graph: start region nodes, copy-only (p = 0).
-inline uint32_t start_min_blocks(uint64_t start_nodes, bool copy_only)
+// The variant for one graph (start region nodes, chance of a direct pick).
+// Measured, one graph a call, against 40 warps with four passes throughout (us):
+//  * a graph below 2^20 nodes is bound by the latency of its dependency chains,
+//    and a step of a chain takes a round of the tile's loop, so tiles of one pass
+//    (n = 10^5, d = 4: 63 -> 53; d = 16: 211 -> 137; n = 10^4, p = 0: 268 -> 115), with
+//    no spills lengthening the round (48 warps: 61; 150; 122);
+//  * up to 2^22 nodes warps count as well (n = 3 * 10^6, d = 16: 833 -> 718; 820 at
+//    32 warps), unless few slots are copies and there is little to wait for
+//    (p = 1: 138 -> 165);
+//  * above, four passes a tile, whose draws overlap and whose first reads go out
+//    together (n = 2^24, d = 4: 978 -> 853; n = 2^28, 64-bit ids: 16,580 -> 15,850; one pass
+//    a tile: 1,085 and 20,800, bound by the claim counters); at p = 1, with no reads,
+//    the 40 warps stay ahead (n = 2^28: 11,424 against 11,740);
+//  * p = 0, every slot a copy and several retries per node, whose passes differ
+//    most in their number of rounds: one pass a tile (n = 2^24: 4,390 -> 3,840).
+inline StartVariant start_variant(uint64_t start_nodes, double p)
 {
-    if (start_nodes < kStartLargeNodes) return kStartMinBlocksSmall;
-    return copy_only ? kStartMinBlocksCopy : kStartMinBlocks;
+    if (start_nodes < (1ull << 20)) return {kStartMinBlocksMid, 1};
+    if (p == 0.0 || (start_nodes < (1ull << 22) && p < 0.75)) return {kStartMinBlocksMany, 1};
+    return {p < 0.95 ? kStartMinBlocksMid : kStartMinBlocks, (uint32_t)kStartPasses};
 }
 
 enum : uint32_t { ST_KNOWN = 0, ST_PEND_GLOBAL = 1, ST_PEND_TILE = 2 };
@@ -485,9 +500,9 @@ struct StartArgs {
 
 // Launch the start kernel; `blocks` 0 = one wave.  The claim counters must be
 // zero and every pair of the graphs' start regions all-ones (fill_start).
-// min_blocks: the variant's resident blocks per SM (start_min_blocks picks it).
-int launch_start(uint32_t id_bytes, const StartArgs &b, uint32_t blocks, cudaStream_t s,
-                 bool slots = false, uint32_t min_blocks = kStartMinBlocks);
+// b.t_end counts tiles of v.passes warp passes (start_variant picks v).
+int launch_start(uint32_t id_bytes, const StartArgs &b, uint32_t blocks, cudaStream_t s, bool slots,
+                 StartVariant v);
 
 // Set every byte of the pairs of nodes [u_first, start_end) of each of `count`
 // graphs to 0xff (one launch).

@@ -508,15 +508,16 @@ int launch_generate(const pa_params *prm, const GenPlan &plan, void *d_edges, vo
         sa.one = a;
         sa.count = 1;
         sa.write_seeds = 1;
-        sa.t_end = plan.start_tiles;
+        const StartVariant variant =
+            start_variant(plan.u_split - plan.u_first, plan.model == PA_MODEL_BA ? 0.5 : prm->p);
+        const uint64_t tile_nodes = (uint64_t)variant.passes * plan.groups;
+        sa.t_end = (plan.u_split - plan.u_first + tile_nodes - 1) / tile_nodes;
         sa.ticket = reinterpret_cast<unsigned long long *>(reinterpret_cast<unsigned char *>(d_scratch) +
                                                           plan.start_offset);
         sa.ctl = a.ctl;
         mrc = mark(1);
         if (mrc != PA_OK) return mrc;
-        const int rc = launch_start(
-            plan.id_bytes, sa, blocks, stream, plan.slots,
-            start_min_blocks(plan.u_split - plan.u_first, plan.pth == 0 && plan.model == PA_MODEL_COPY));
+        const int rc = launch_start(plan.id_bytes, sa, blocks, stream, plan.slots, variant);
         if (rc != PA_OK) return rc;
         if (plan.u_split >= prm->n) {
             mrc = mark(2);

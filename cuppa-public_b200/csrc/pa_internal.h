@@ -44,7 +44,7 @@ constexpr uint32_t kTraceMax = 2048; // progress samples kept per generation
 // the start kernel's claim counters: 8, a 128-byte line each
 constexpr uint64_t kStartAreaBytes = 1024;
 
-// Warp passes per start tile, the start kernel's unit of work.
+// Warp passes per start tile, the start kernel's unit of work, where it is not one.
 constexpr int kStartPasses = 4;
 
 // Resolved launch geometry of one generation.
@@ -59,7 +59,6 @@ struct GenPlan {
     uint64_t sb_offset;     // byte offset of the superblock counters in the scratch
     uint64_t trace_offset;  // byte offset of the progress trace in the scratch
     uint64_t start_offset;  // byte offset of the start kernel's counters
-    uint64_t start_tiles;   // start tiles of the start region
     uint64_t u_split;       // nodes [u_first, u_split) are the start kernel's
     uint32_t claim_tiles;   // tiles (or start tiles) per claim-counter atomic
     uint64_t seed_edges;

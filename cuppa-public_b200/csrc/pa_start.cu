@@ -24,9 +24,12 @@
 // readers -- measured slower on B200 than the memset it saves: 88.7 against
 // 68.0 ms for n = 2^30, d = 4.)
 //
-// Work is claimed one start tile at a time: kStartPasses warp passes of G =
-// 32/d nodes each (lane = node-in-pass * d + slot), resolved together, so a
-// wait in one pass does not hold back the others.  Warp w of a block claims
+// Work is claimed one start tile at a time: P warp passes (one or kStartPasses,
+// start_variant says which and why) of G = 32/d nodes each (lane = node-in-pass
+// * d + slot), resolved together, so a wait in one pass does not hold back the
+// others.  Claims of several tiles at once were tried for one-pass tiles: a tile
+// behind an unfinished one of its warp holds up every chain through it (n =
+// 10^6, d = 4, eight a claim: 379 against 107 us).  Warp w of a block claims
 // from counter w (of kStartCounters), which hands out tiles w, w + 8, ... in
 // increasing order: eight counter lines instead of one, since a single counter
 // saturates at one atomic every few nanoseconds.  Several graphs share one
@@ -64,36 +67,45 @@ __device__ __forceinline__ bool read_slot(Slot<uint32_t> &s, const GenArgs &a, c
 }
 
 // Where the candidate of a fresh draw comes from (32-bit node arithmetic: the
-// start region ends below 2^31).
+// start region ends below 2^31); true if slot (s.val, k) is to be read for it.
+__device__ __forceinline__ bool place_start(Slot<uint32_t> &s, const DrawT<uint32_t> &dr, uint32_t r,
+                                            const GenArgs &a, uint32_t pbase)
+{
+    uint32_t st = ST_KNOWN;
+    s.val = dr.v;
+    bool read = false;
+    if (!dr.direct) {
+        if (dr.v <= a.d) {
+            s.val = (uint32_t)seed_slot(dr.v, dr.k, a.d, a.seed_mode);
+        } else if (dr.v < pbase) {
+            read = true;
+        } else {
+            st = ST_PEND_TILE;   // an earlier node of this same pass
+        }
+    }
+    s.meta = st | (dr.k << 2) | (r << 8);
+    return read;
+}
+
 template <typename Id, bool Slots>
 __device__ __forceinline__ void classify_start(Slot<uint32_t> &s, const DrawT<uint32_t> &dr,
                                                uint32_t r, const GenArgs &a, const Id *E,
                                                uint32_t pbase, uint32_t &n_pend)
 {
-    uint32_t st = ST_KNOWN;
-    if (dr.direct) {
-        s.val = dr.v;
-    } else if (dr.v <= a.d) {
-        s.val = (uint32_t)seed_slot(dr.v, dr.k, a.d, a.seed_mode);
-    } else if (dr.v < pbase) {
-        if (!read_slot<Id, Slots>(s, a, E, dr.v, dr.k)) {
-            st = ST_PEND_GLOBAL;
-            ++n_pend;
-        }
-    } else {
-        s.val = dr.v;   // an earlier node of this same pass
-        st = ST_PEND_TILE;
+    if (place_start(s, dr, r, a, pbase) &&
+        !read_slot<Id, Slots>(s, a, E, s.val, meta_k(s.meta))) {
+        s.meta |= ST_PEND_GLOBAL;
+        ++n_pend;
     }
-    s.meta = st | (dr.k << 2) | (r << 8);
 }
 
-// Resolve the kStartPasses warp passes of one start tile together; every slot is
+// Resolve the P warp passes of one start tile together; every slot is
 // stored as soon as it is final.  Copy sources in the lane's own pass come from
 // the source lane by shuffle; sources in an earlier pass of the tile are polled
 // in memory like any other.  Returns false when the warp must stop (wait limit,
 // or another warp failed).
-template <typename Id, bool Slots>
-__device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[kStartPasses], const GenArgs &a,
+template <typename Id, bool Slots, int P>
+__device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[P], const GenArgs &a,
                                               Id *E, uint32_t tb, bool withhold, const Lane &L,
                                               uint32_t &n_retry, uint32_t &n_wait,
                                               uint32_t &n_pend, uint32_t &n_poll)
@@ -104,7 +116,7 @@ __device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[kStartPasses],
     Id *pair0 = Slots ? E + e_lane : E + 2 * e_lane;
     uint32_t stored = 0;   // bit j: pass j's slot is stored (or inactive)
 #pragma unroll
-    for (int j = 0; j < kStartPasses; ++j)
+    for (int j = 0; j < P; ++j)
         if (!(L.used && tb + j * G + L.g < a.start_end)) stored |= 1u << j;
     const uint32_t max_sleep = min(a.max_sleep_ns, 512u);
     uint64_t spin_t0 = 0;
@@ -115,11 +127,11 @@ __device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[kStartPasses],
     // bit j: this lane's slot of pass j changed after the pass's last match; a
     // pass in which no lane changed would match and vote exactly as before, so
     // only its pending reads are polled (one vote per pass and round)
-    uint32_t dirty = (1u << kStartPasses) - 1u;
+    uint32_t dirty = (1u << P) - 1u;
     for (;;) {
         bool changed = false;
 #pragma unroll
-        for (int j = 0; j < kStartPasses; ++j) {
+        for (int j = 0; j < P; ++j) {
             if ((done >> j) & 1u) continue;
             const uint32_t pbase = tb + j * G;
             const uint32_t u = pbase + L.g;
@@ -176,7 +188,7 @@ __device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[kStartPasses],
                 ++n_retry;
             }
         }
-        if (done == (1u << kStartPasses) - 1u) return true;
+        if (done == (1u << P) - 1u) return true;
 
         if (!__any_sync(kFull, changed)) {
             unsigned long long now = 0;
@@ -211,7 +223,7 @@ __device__ __forceinline__ void set_lane(Lane &L, const GenArgs &a)
     L.gmask = L.used ? (a.d == 32 ? kFull : (((1u << a.d) - 1u) << (L.g * a.d))) : 0u;
 }
 
-template <typename Id, bool Slots, uint32_t MinBlocks>
+template <typename Id, bool Slots, uint32_t MinBlocks, int P>
 __global__ void __launch_bounds__(kThreads, MinBlocks) start_kernel(const StartArgs b)
 {
     __shared__ GenArgs s_args[kThreads / 32];
@@ -302,20 +314,53 @@ __global__ void __launch_bounds__(kThreads, MinBlocks) start_kernel(const StartA
             set_lane(L, a);
         }
         Id *E = reinterpret_cast<Id *>(a.edges);
-        const uint32_t tb = (uint32_t)(a.u_first + t * (kStartPasses * a.groups));
-        Slot<uint32_t> s[kStartPasses];
+        const uint32_t tb = (uint32_t)(a.u_first + t * (P * a.groups));
+        Slot<uint32_t> s[P];
+        if constexpr (P == 1 || MinBlocks != kStartMinBlocksMid) {
 #pragma unroll
-        for (int j = 0; j < kStartPasses; ++j) {
-            const uint32_t pbase = tb + j * a.groups;
-            const uint32_t u = pbase + L.g;
-            s[j].val = 0;
-            s[j].meta = ST_KNOWN;
-            if (L.used && u < a.start_end)
-                classify_start<Id, Slots>(s[j], draw<uint32_t>(u, L.slot, 0u, a), 0u, a, E, pbase,
-                                          n_pend);
+            for (int j = 0; j < P; ++j) {
+                const uint32_t pbase = tb + j * a.groups;
+                const uint32_t u = pbase + L.g;
+                s[j].val = 0;
+                s[j].meta = ST_KNOWN;
+                if (L.used && u < a.start_end)
+                    classify_start<Id, Slots>(s[j], draw<uint32_t>(u, L.slot, 0u, a), 0u, a, E,
+                                              pbase, n_pend);
+            }
+        } else {
+            // the passes' first reads go out together, so that a tile waits for one
+            // memory latency and not for one per pass
+            uint32_t x[P];
+            uint32_t reads = 0;   // bit j: pass j's slot of this lane is read
+#pragma unroll
+            for (int j = 0; j < P; ++j) {
+                const uint32_t pbase = tb + j * a.groups;
+                const uint32_t u = pbase + L.g;
+                s[j].val = 0;
+                s[j].meta = ST_KNOWN;
+                if (L.used && u < a.start_end &&
+                    place_start(s[j], draw<uint32_t>(u, L.slot, 0u, a), 0u, a, pbase))
+                    reads |= 1u << j;
+            }
+#pragma unroll
+            for (int j = 0; j < P; ++j)
+                if ((reads >> j) & 1u)
+                    x[j] = (uint32_t)ld_slot(
+                        slot_addr<Id, uint32_t, Slots>(E, a, s[j].val, meta_k(s[j].meta)));
+#pragma unroll
+            for (int j = 0; j < P; ++j)
+                if ((reads >> j) & 1u) {
+                    // values are below 2^31: the low word tells the fill
+                    if (x[j] != 0xffffffffu) {
+                        s[j].val = x[j];
+                    } else {
+                        s[j].meta |= ST_PEND_GLOBAL;
+                        ++n_pend;
+                    }
+                }
         }
-        ok = resolve_start<Id, Slots>(s, a, E, tb, a.withhold_first && t == 0, L, n_retry, n_wait, n_pend,
-                               n_poll);
+        ok = resolve_start<Id, Slots, P>(s, a, E, tb, a.withhold_first && t == 0, L, n_retry, n_wait,
+                                         n_pend, n_poll);
     }
 
 #pragma unroll
@@ -362,10 +407,10 @@ __global__ void fill_start_kernel(const GenArgs *inst, uint32_t y0, uint32_t id_
         p[x] = ones;
 }
 
-template <typename Id, bool Slots, uint32_t MinBlocks>
+template <typename Id, bool Slots, uint32_t MinBlocks, int P>
 int launch_start_t(const StartArgs &b, uint32_t blocks, cudaStream_t s)
 {
-    auto kern = start_kernel<Id, Slots, MinBlocks>;
+    auto kern = start_kernel<Id, Slots, MinBlocks, P>;
     if (blocks == 0) {
         int dev = 0, sms = 0, per_sm = 0;
         cudaError_t e = cudaGetDevice(&dev);
@@ -386,25 +431,27 @@ int launch_start_t(const StartArgs &b, uint32_t blocks, cudaStream_t s)
 
 }  // namespace
 
-template <uint32_t MinBlocks>
+template <uint32_t MinBlocks, int P>
 int launch_start_m(uint32_t id_bytes, const StartArgs &b, uint32_t blocks, cudaStream_t s,
                    bool slots)
 {
     if (slots)
-        return id_bytes == 8 ? launch_start_t<int64_t, true, MinBlocks>(b, blocks, s)
-                             : launch_start_t<int32_t, true, MinBlocks>(b, blocks, s);
-    return id_bytes == 8 ? launch_start_t<int64_t, false, MinBlocks>(b, blocks, s)
-                         : launch_start_t<int32_t, false, MinBlocks>(b, blocks, s);
+        return id_bytes == 8 ? launch_start_t<int64_t, true, MinBlocks, P>(b, blocks, s)
+                             : launch_start_t<int32_t, true, MinBlocks, P>(b, blocks, s);
+    return id_bytes == 8 ? launch_start_t<int64_t, false, MinBlocks, P>(b, blocks, s)
+                         : launch_start_t<int32_t, false, MinBlocks, P>(b, blocks, s);
 }
 
 int launch_start(uint32_t id_bytes, const StartArgs &b, uint32_t blocks, cudaStream_t s,
-                 bool slots, uint32_t min_blocks)
+                 bool slots, StartVariant v)
 {
-    if (min_blocks == kStartMinBlocksCopy)
-        return launch_start_m<kStartMinBlocksCopy>(id_bytes, b, blocks, s, slots);
-    if (min_blocks == kStartMinBlocksSmall)
-        return launch_start_m<kStartMinBlocksSmall>(id_bytes, b, blocks, s, slots);
-    return launch_start_m<kStartMinBlocks>(id_bytes, b, blocks, s, slots);
+    if (v.passes == 1)
+        return v.min_blocks == kStartMinBlocksMany
+                   ? launch_start_m<kStartMinBlocksMany, 1>(id_bytes, b, blocks, s, slots)
+                   : launch_start_m<kStartMinBlocksMid, 1>(id_bytes, b, blocks, s, slots);
+    if (v.min_blocks == kStartMinBlocksMid)
+        return launch_start_m<kStartMinBlocksMid, kStartPasses>(id_bytes, b, blocks, s, slots);
+    return launch_start_m<kStartMinBlocks, kStartPasses>(id_bytes, b, blocks, s, slots);
 }
 
 int fill_start(uint32_t id_bytes, const GenArgs *d_inst, uint32_t count, uint64_t max_pairs,

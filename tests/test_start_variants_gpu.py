@@ -1,0 +1,37 @@
+"""The start kernel's variants (one or four warp passes per tile, 32, 40 or 48
+warps per SM), chosen by the number of nodes and the chance of a direct pick: sizes on
+both sides of the lines (2^20 and 2^22 nodes), last tiles cut short, both layouts and id
+widths, d with idle lanes, against the oracle."""
+import numpy as np
+import pytest
+
+import _oracle as orc
+
+pytestmark = pytest.mark.gpu
+
+EDGE = [(2 ** 20 + d + 1 + x, d) for d in (1, 3) for x in (-1, 0, 1)] + \
+       [(2 ** 22 + d + 1 + x, d) for d in (1, 2) for x in (-1, 0, 5)]
+
+
+@pytest.mark.parametrize("p", [0.0, 0.3, 0.8, 1.0])
+@pytest.mark.parametrize("n,d", EDGE)
+def test_variants_match_oracle(pa, cuda_ok, n, d, p):
+    slots = (n + d) % 2
+    bits = 64 if n % 3 == 0 else 32
+    prm = pa.make_params(n, d, p, seed=n, id_bits=bits, layout=slots)
+    edges, st = pa.generate(prm)
+    G, retries = orc.generate(n, d, p, n, orc.SEED_CLIQUE, with_retries=True)
+    assert st.retries == retries
+    got = edges.cpu().numpy()
+    want = G[d + 1:] if slots else orc.pairs_slot_order(G, orc.SEED_CLIQUE)
+    assert (got.astype(np.int64) == want).all()
+
+
+def test_ba_above_the_lines(pa, cuda_ok):
+    for n in (2 ** 20 + 9, 2 ** 22 + 9):
+        prm = pa.make_params(n, 2, 0.0, seed=5, id_bits=64, seed_mode=pa.PA_SEED_STAR_REF,
+                             model=pa.PA_MODEL_BA)
+        edges, st = pa.generate(prm)
+        G, retries = orc.generate_ba(n, 2, 5, with_retries=True)
+        assert st.retries == retries
+        assert (edges.cpu().numpy() == orc.pairs_slot_order(G, orc.SEED_STAR_REF)).all()
