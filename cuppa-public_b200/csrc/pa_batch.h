@@ -28,8 +28,9 @@ struct BatchJob {
     gen::GenArgs first{};                      // instance 0 (the start kernel's count == 1 path)
 };
 
-// Validate prms and lay out the scratch (J.scratch_bytes, J.image_bytes).
-int batch_prepare(const pa_params *prms, uint32_t count, BatchJob &J);
+// Validate prms and lay out the scratch (J.scratch_bytes, J.image_bytes).  coarse:
+// larger first levels, smaller tables.
+int batch_prepare(const pa_params *prms, uint32_t count, BatchJob &J, bool coarse = false);
 // Write the image (J.image_bytes) for these edge buffers and this scratch.
 int batch_bind(BatchJob &J, const pa_params *prms, void *const *d_edges, const uint64_t *edges_bytes,
                void *d_scratch, unsigned char *image);

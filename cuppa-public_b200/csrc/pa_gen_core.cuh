@@ -422,8 +422,14 @@ __device__ __forceinline__ bool stage2(Slot<NodeT> (&s)[P], uint64_t t, const Ge
 namespace pa {
 namespace gen {
 
-constexpr uint64_t kLevelMinNodes = 4096;
-constexpr uint32_t kLevelShift = 3;
+// Nodes of the first levels, and their growth.  A level's units of one graph
+// follow one another, so warps that take a large first level work on few graphs at
+// a time, each bound by the latency of its dependency chains: first levels of
+// 4,096 nodes growing by 1/8 took 17.4 ms for 512 graphs of 10^3..10^5 nodes,
+// these 6.7 (64 nodes: 6.4, with more levels to keep and search); 256 graphs of
+// 10^3..10^6 nodes 15.9 -> 10.5 ms, 64 of 10^3..10^7 20.3 -> 18.8.
+constexpr uint64_t kLevelMinNodes = 128, kLevelMinNodesCoarse = 4096;
+constexpr uint32_t kLevelShift = 2, kLevelShiftCoarse = 3;
 constexpr uint32_t kMaxLevels = 160;
 
 // Device copies of the level tables of a set of graphs.
@@ -436,8 +442,8 @@ struct LevelTables {
 
 // Unit bounds of a graph's levels over nodes [u_first, n_end) in units of
 // unit_nodes: entry l is the first unit of level l, the last is n_units.
-std::vector<uint64_t> level_bounds(uint64_t u_first, uint64_t n_end, uint64_t n_units,
-                                   uint64_t unit_nodes);
+std::vector<uint64_t> level_bounds(uint64_t u_first, uint64_t lo, uint64_t n_end,
+                                   uint64_t unit_nodes, bool coarse);
 
 // Largest index i in [0, len) with a[i] <= x (a ascending, a[0] <= x).
 __device__ __forceinline__ uint32_t last_le(const unsigned long long *a, uint32_t len,

@@ -459,7 +459,10 @@ int fill_start(uint32_t id_bytes, const GenArgs *d_inst, uint32_t count, uint64_
 {
     if (count == 0 || max_pairs == 0) return PA_OK;
     const uint64_t n16 = max_pairs * 2ull * id_bytes / 16 + 1;
-    const uint32_t gx = (uint32_t)std::min<uint64_t>(4096, (n16 + 255) / 256);
+    // 16 stores a thread for the largest graph: with one, the blocks of many small
+    // graphs, most of them with nothing to do, took longer than the stores (a call
+    // of 512 graphs of 10^3..10^5 nodes 6.7 -> 5.5 ms)
+    const uint32_t gx = (uint32_t)std::min<uint64_t>(4096, (n16 + 4095) / 4096);
     for (uint32_t y0 = 0; y0 < count; y0 += 65535) {
         const uint32_t gy = std::min<uint32_t>(65535, count - y0);
         fill_start_kernel<<<dim3(gx, gy), 256, 0, s>>>(d_inst, y0, id_bytes);

@@ -35,3 +35,30 @@ def test_ba_above_the_lines(pa, cuda_ok):
         G, retries = orc.generate_ba(n, 2, 5, with_retries=True)
         assert st.retries == retries
         assert (edges.cpu().numpy() == orc.pairs_slot_order(G, orc.SEED_STAR_REF)).all()
+
+
+def test_batch_in_the_scratch_of_coarse_levels(pa, cuda_ok):
+    """A caller's scratch too small for the tables of many small levels gets fewer
+    levels and the same graphs; one too small for those is refused."""
+    import ctypes
+    import torch
+    prms = [pa.make_params(n, d, 0.4, seed=i) for i, (n, d) in
+            enumerate([(30000, 4), (1000, 32), (70001, 3), (9, 8), (5000, 17)])]
+    b = pa.Batch(prms)
+    b.generate()
+    assert b.finish().status == 0
+    want = [b.graph(i).clone() for i in range(len(prms))]
+    full, least = b.scratch.numel(), None
+    for size in range(full, 0, -256):
+        b.scratch = torch.empty(size, dtype=torch.uint8, device="cuda")
+        for i in range(len(prms)):
+            b.graph(i).zero_()
+        try:
+            b.generate()
+        except pa.CuppaError as e:
+            assert e.status == pa.PA_ERR_CAPACITY
+            break
+        least = size
+        assert b.finish().status == 0
+        assert all(torch.equal(b.graph(i), w) for i, w in enumerate(want))
+    assert least is not None and least < full
