@@ -24,13 +24,6 @@
 
 #include "pa_batch.h"
 
-// Resident start-kernel blocks per SM of a batch launch (a variant of four passes
-// per tile: 4 or 5; the 64-graph mix of 10^3..10^7 nodes 21.3 -> 20.3 ms at 4, one pass
-// per tile 26.8-29.0, bound by the claim counters).
-#ifndef PA_BATCH_START_BLOCKS
-#define PA_BATCH_START_BLOCKS gen::kStartMinBlocksMid
-#endif
-
 namespace pa {
 namespace gen {
 
@@ -249,6 +242,7 @@ int batch_prepare(const pa_params *prms, uint32_t count, BatchJob &J, bool coars
     J.flags_off.assign(count, 0);
     J.sb_off.assign(count, 0);
     std::vector<std::vector<uint64_t>> sb(count), tb(count);
+    uint64_t slots = 0;
     for (uint32_t i = 0; i < count; ++i) {
         pa_params q = prms[i];
         q.tile_passes = P;   // one pass count per launch
@@ -259,10 +253,15 @@ int batch_prepare(const pa_params *prms, uint32_t count, BatchJob &J, bool coars
         if (prms[i].id_bits != prms[0].id_bits) return PA_ERR_INVALID;
         if (prms[i].n + p.tile_nodes + 32 >= (1ull << 32)) return PA_ERR_NOT_SUPPORTED;
         if (prms[i].flags != 0) return PA_ERR_INVALID;
-        sb[i] = level_bounds(p.u_first, p.u_first, p.u_split, (uint64_t)kStartPasses * p.groups,
+        J.max_start_pairs = std::max<uint64_t>(J.max_start_pairs, (p.u_split - p.u_first) * prms[i].d);
+        slots += (p.u_split - p.u_first) * prms[i].d;
+    }
+    J.variant = gen::batch_variant(slots);
+    for (uint32_t i = 0; i < count; ++i) {
+        const GenPlan &p = J.plans[i];
+        sb[i] = level_bounds(p.u_first, p.u_first, p.u_split, (uint64_t)J.variant.passes * p.groups,
                              coarse);
         tb[i] = level_bounds(p.u_first, p.u_split, prms[i].n, p.tile_nodes, coarse);
-        J.max_start_pairs = std::max<uint64_t>(J.max_start_pairs, (p.u_split - p.u_first) * prms[i].d);
     }
     build_levels(sb, J.start);
     build_levels(tb, J.tail);
@@ -370,7 +369,7 @@ int batch_enqueue(const BatchJob &J, void *d_scratch, const void *image, cudaStr
     sa.ctl = ctl;
     if (J.count == 1) sa.one = J.first;
     rc = gen::launch_start(J.id_bytes, sa, 0, s, false,
-                           gen::StartVariant{PA_BATCH_START_BLOCKS, (uint32_t)kStartPasses});
+                           J.variant);
     if (rc != PA_OK) return rc;
     return gen::launch_tail(J.id_bytes, J.passes, d_inst, device_tables(J.tail, scr), J.count,
                             J.tail.lvl[0], J.tail.lvl[J.tail.levels], tail_ticket, ctl,

@@ -24,6 +24,7 @@ struct BatchJob {
     BatchLevels start, tail;
     uint64_t image_off = 0, image_bytes = 0;   // scratch bytes copied from the host image
     uint64_t table_off = 0, ticket_off = 0, scratch_bytes = 0;
+    gen::StartVariant variant{};               // of the start launch
     uint64_t max_start_pairs = 0;       // the largest start region (fill launch size)
     gen::GenArgs first{};                      // instance 0 (the start kernel's count == 1 path)
 };

@@ -36,8 +36,9 @@ struct StartVariant {
 //  * up to 2^22 nodes warps count as well (n = 3 * 10^6, d = 16: 833 -> 718; 820 at
 //    32 warps), unless few slots are copies and there is little to wait for
 //    (p = 1: 138 -> 165);
-//  * above, four passes a tile, whose draws overlap and whose first reads go out
-//    together (n = 2^24, d = 4: 978 -> 853; n = 2^28, 64-bit ids: 16,580 -> 15,850; one pass
+//  * above, two, then four passes a tile, whose draws overlap and whose first reads
+//    go out together (n = 5 * 10^6, d = 7, p = 0.3: 696 -> 600 with two passes at 40 warps;
+//    n = 2^24, d = 4: 978 -> 853; n = 2^28, 64-bit ids: 16,580 -> 15,850; one pass
 //    a tile: 1,085 and 20,800, bound by the claim counters); at p = 1, with no reads,
 //    the 40 warps stay ahead (n = 2^28: 11,424 against 11,740);
 //  * p = 0, every slot a copy and several retries per node, whose passes differ
@@ -46,7 +47,18 @@ inline StartVariant start_variant(uint64_t start_nodes, double p)
 {
     if (start_nodes < (1ull << 20)) return {kStartMinBlocksMid, 1};
     if (p == 0.0 || (start_nodes < (1ull << 22) && p < 0.75)) return {kStartMinBlocksMany, 1};
+    if (start_nodes <= (1ull << 24) && p < 0.75) return {kStartMinBlocks, 2};
     return {p < 0.95 ? kStartMinBlocksMid : kStartMinBlocks, (uint32_t)kStartPasses};
+}
+
+// The variant for a batch of graphs with `slots` slots: chains of a small batch
+// leave warps waiting, as in a single graph (8 graphs of 10^4..10^5 nodes: 630 us
+// at four passes, 528 at two; 512 of 10^3..10^5, 185M slots: 5.55 and 5.99 ms; one
+// pass, bound by the claim counters: 64 of 10^3..10^7 26.8 ms, 18.8 at four).
+inline StartVariant batch_variant(uint64_t slots)
+{
+    if (slots < (1ull << 25)) return {kStartMinBlocks, 2};
+    return {kStartMinBlocksMid, (uint32_t)kStartPasses};
 }
 
 enum : uint32_t { ST_KNOWN = 0, ST_PEND_GLOBAL = 1, ST_PEND_TILE = 2 };

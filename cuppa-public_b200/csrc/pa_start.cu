@@ -24,7 +24,7 @@
 // readers -- measured slower on B200 than the memset it saves: 88.7 against
 // 68.0 ms for n = 2^30, d = 4.)
 //
-// Work is claimed one start tile at a time: P warp passes (one or kStartPasses,
+// Work is claimed one start tile at a time: P warp passes (1, 2 or kStartPasses,
 // start_variant says which and why) of G = 32/d nodes each (lane = node-in-pass
 // * d + slot), resolved together, so a wait in one pass does not hold back the
 // others.  Claims of several tiles at once were tried for one-pass tiles: a tile
@@ -316,7 +316,7 @@ __global__ void __launch_bounds__(kThreads, MinBlocks) start_kernel(const StartA
         Id *E = reinterpret_cast<Id *>(a.edges);
         const uint32_t tb = (uint32_t)(a.u_first + t * (P * a.groups));
         Slot<uint32_t> s[P];
-        if constexpr (P == 1 || MinBlocks != kStartMinBlocksMid) {
+        if constexpr (P == 1 || (P == kStartPasses && MinBlocks == kStartMinBlocks)) {
 #pragma unroll
             for (int j = 0; j < P; ++j) {
                 const uint32_t pbase = tb + j * a.groups;
@@ -449,6 +449,7 @@ int launch_start(uint32_t id_bytes, const StartArgs &b, uint32_t blocks, cudaStr
         return v.min_blocks == kStartMinBlocksMany
                    ? launch_start_m<kStartMinBlocksMany, 1>(id_bytes, b, blocks, s, slots)
                    : launch_start_m<kStartMinBlocksMid, 1>(id_bytes, b, blocks, s, slots);
+    if (v.passes == 2) return launch_start_m<kStartMinBlocks, 2>(id_bytes, b, blocks, s, slots);
     if (v.min_blocks == kStartMinBlocksMid)
         return launch_start_m<kStartMinBlocksMid, kStartPasses>(id_bytes, b, blocks, s, slots);
     return launch_start_m<kStartMinBlocks, kStartPasses>(id_bytes, b, blocks, s, slots);

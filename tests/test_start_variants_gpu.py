@@ -1,6 +1,6 @@
-"""The start kernel's variants (one or four warp passes per tile, 32, 40 or 48
+"""The start kernel's variants (1, 2 or 4 warp passes per tile, 32, 40 or 48
 warps per SM), chosen by the number of nodes and the chance of a direct pick: sizes on
-both sides of the lines (2^20 and 2^22 nodes), last tiles cut short, both layouts and id
+both sides of the lines (2^20, 2^22 and 2^24 nodes), last tiles cut short, both layouts and id
 widths, d with idle lanes, against the oracle."""
 import numpy as np
 import pytest
@@ -10,7 +10,8 @@ import _oracle as orc
 pytestmark = pytest.mark.gpu
 
 EDGE = [(2 ** 20 + d + 1 + x, d) for d in (1, 3) for x in (-1, 0, 1)] + \
-       [(2 ** 22 + d + 1 + x, d) for d in (1, 2) for x in (-1, 0, 5)]
+       [(2 ** 22 + d + 1 + x, d) for d in (1, 2) for x in (-1, 0, 5)] + \
+       [(2 ** 24 + 2 + x, 1) for x in (0, 1)]
 
 
 @pytest.mark.parametrize("p", [0.0, 0.3, 0.8, 1.0])
