@@ -25,10 +25,11 @@
 // The draws (Philox counter (u_lo, u_hi, slot, retry)), the slot order and the
 // rejection rule are the start kernel's, so the output is bit-identical to the
 // sequential definition (src/PA/SPA/SerialCopyModel3.cpp:52-78 with Philox
-// draws) for any d.  Nodes are claimed in increasing order from one counter; a
-// warp holds one node and waits only on lower nodes, so the lowest unfinished
-// node always progresses, for any grid.  Every wait is bounded by
-// spin_limit_ns.
+// draws) for any d.  Warp w of a block of W claims nodes w, w + W, ... in increasing
+// order from counter w; a warp holds one node and waits only on lower nodes, and
+// any resident block has a warp on every counter, so the lowest unfinished node is
+// held, or next on a counter whose warps are free: it always progresses, for any
+// grid.  Every wait is bounded by spin_limit_ns.
 //
 // Also here: canonical rows and CSR out parts of such graphs (each row ranked
 // by one warp from a copy in shared memory), for d <= kWideRankMaxD.
@@ -152,7 +153,7 @@ __device__ __forceinline__ void wide_prefetch(uint32_t *pre_val, uint32_t *pre_m
     }
 }
 
-template <typename Id, bool Slots>
+template <typename Id, bool Slots, bool Skip>
 __global__ void wide_kernel(const GenArgs a, unsigned long long *ticket, uint32_t cap_log2,
                             uint32_t write_seeds, uint32_t prefetch)
 {
@@ -168,8 +169,9 @@ __global__ void wide_kernel(const GenArgs a, unsigned long long *ticket, uint32_
     const uint32_t lt = lanemask_lt(), le = lt | (1u << lane);
     const uint32_t d = a.d;
     Id *E = reinterpret_cast<Id *>(a.edges);
-    const uint32_t gw = blockIdx.x * (blockDim.x >> 5) + warp;
-    const uint32_t nw = gridDim.x * (blockDim.x >> 5);
+    const uint32_t warps = blockDim.x >> 5;
+    const uint32_t gw = blockIdx.x * warps + warp;
+    const uint32_t nw = gridDim.x * warps;
 
     if (!Slots && write_seeds) {
         for (uint64_t e = (uint64_t)gw * 32 + lane; e < a.seed_edges; e += (uint64_t)nw * 32) {
@@ -183,13 +185,15 @@ __global__ void wide_kernel(const GenArgs a, unsigned long long *ticket, uint32_
     const uint32_t max_sleep = min(a.max_sleep_ns, 512u);
     bool ok = true;
     while (ok) {
+        // counter `warp` hands out nodes warp, warp + warps, ... in increasing order
+        // (any resident block has a warp on every counter): one counter saturates at
+        // an atomic every few nanoseconds
         unsigned long long c = 0;
-        if (lane == 0) c = atomicAdd(ticket, 1ull);
-        c = __shfl_sync(kFull, c, 0);
-        const uint64_t u64 = a.u_first + c;
+        if (lane == 0) c = atomicAdd(ticket + 16 * warp, 1ull);
+        const uint64_t row = __shfl_sync(kFull, c, 0) * warps + warp;
+        const uint64_t u64 = a.u_first + row;
         if (u64 >= a.start_end) break;
         const uint32_t u = (uint32_t)u64;
-        const uint64_t row = c;
         const bool withhold = a.withhold_first && row == 0;
         __syncwarp();
         for (uint32_t x = lane; x < cap; x += 32) set[x] = kEmpty;
@@ -208,6 +212,11 @@ __global__ void wide_kernel(const GenArgs a, unsigned long long *ticket, uint32_
                 wide_classify<Id, Slots>(s, u, i, 0u, a, E, n_pend);
             }
             bool stored = !active;
+            // After a round that changed nothing (work = false) a round in which no
+            // lane's candidate is new would match as that one did: warps that only
+            // wait leave the match unit, shared by the SM, to those that do not (n =
+            // 5,000, d = 100, p = 0.4: 1,510 -> 1,215 us).
+            bool fresh = true, work = true;
             const uint64_t e = a.seed_edges + row * d + i;
             uint64_t spin_t0 = 0;
             uint32_t sleep_ns = 32;
@@ -219,38 +228,44 @@ __global__ void wide_kernel(const GenArgs a, unsigned long long *ticket, uint32_
                         s.val = (uint32_t)x;
                         s.known = true;
                         changed = true;
+                        fresh = true;
                     } else {
                         ++n_poll;
                     }
                 }
-                // a candidate among the earlier chunks' final values is rejected
-                // now, as often as it takes (every value in the set is final)
-                while (active && s.known && set_contains(set, cap_log2, s.val)) {
-                    wide_classify<Id, Slots>(s, u, i, s.r + 1u, a, E, n_pend);
-                    ++n_retry;
-                    changed = true;
-                }
-                const bool known = active && s.known;
-                const uint32_t eq = __match_any_sync(kFull, known ? s.val : (0xffffffe0u | lane));
-                const bool bad = active && (!known || (eq & lt) != 0u);
-                const uint32_t badm = __ballot_sync(kFull, bad);
-                const bool fin = active && (badm & le) == 0u;
-                if (fin && !stored) {
-                    if (!withhold) {
-                        if constexpr (Slots) st_relaxed_id(E + e, s.val);
-                        else st_relaxed_pair(E + 2 * e, u, s.val);
+                if (!Skip || work || __any_sync(kFull, fresh)) {
+                    // a candidate among the earlier chunks' final values is rejected
+                    // now, as often as it takes (every value in the set is final)
+                    while (active && s.known && set_contains(set, cap_log2, s.val)) {
+                        wide_classify<Id, Slots>(s, u, i, s.r + 1u, a, E, n_pend);
+                        ++n_retry;
+                        changed = true;
                     }
-                    stored = true;
+                    fresh = false;
+                    const bool known = active && s.known;
+                    const uint32_t eq = __match_any_sync(kFull, known ? s.val : (0xffffffe0u | lane));
+                    const bool bad = active && (!known || (eq & lt) != 0u);
+                    const uint32_t badm = __ballot_sync(kFull, bad);
+                    const bool fin = active && (badm & le) == 0u;
+                    if (fin && !stored) {
+                        if (!withhold) {
+                            if constexpr (Slots) st_relaxed_id(E + e, s.val);
+                            else st_relaxed_pair(E + 2 * e, u, s.val);
+                        }
+                        stored = true;
+                    }
+                    const uint32_t finm = __ballot_sync(kFull, fin || !active);
+                    if (finm == kFull) break;
+                    // a candidate equal to a final lower slot of the chunk is rejected
+                    if (known && !fin && (eq & lt & finm) != 0u) {
+                        wide_classify<Id, Slots>(s, u, i, s.r + 1u, a, E, n_pend);
+                        ++n_retry;
+                        changed = true;
+                        fresh = true;
+                    }
                 }
-                const uint32_t finm = __ballot_sync(kFull, fin || !active);
-                if (finm == kFull) break;
-                // a candidate equal to a final lower slot of the chunk is rejected
-                if (known && !fin && (eq & lt & finm) != 0u) {
-                    wide_classify<Id, Slots>(s, u, i, s.r + 1u, a, E, n_pend);
-                    ++n_retry;
-                    changed = true;
-                }
-                if (!__any_sync(kFull, changed)) {
+                work = __any_sync(kFull, changed);
+                if (!work) {
                     unsigned long long now = 0;
                     uint32_t err = 0;
                     if (lane == 0) {
@@ -318,7 +333,9 @@ int launch_wide_t(const GenArgs &a, unsigned long long *ticket, uint32_t blocks,
     const uint32_t warps = (uint32_t)std::max<size_t>(
         1, std::min<size_t>(8, kWideBlockSetBytes / warp_bytes));
     const size_t smem = warp_bytes * warps;
-    auto kern = wide_kernel<Id, Slots>;
+    // an SM with one or two such warps has a match unit to spare (d = 4,000: 390 ms,
+    // 402 with the votes that skip it)
+    auto kern = warps > 2 ? wide_kernel<Id, Slots, true> : wide_kernel<Id, Slots, false>;
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return set_cuda_error(e);
     if (blocks == 0) {

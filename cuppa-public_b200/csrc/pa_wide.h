@@ -18,7 +18,8 @@ constexpr size_t kWideBlockSetBytes = 64 * 1024;
 constexpr uint32_t kWideSetMaxBytes = 128 * 1024;
 
 // Generate nodes [a.u_first, a.start_end) of a graph with d > 32 into caller
-// memory whose slots of those nodes hold all-ones; *ticket must be zero.  Also
+// memory whose slots of those nodes hold all-ones; the claim counters (eight, 128
+// bytes apart) must be zero.  Also
 // writes the seed edges (PAIRS).  `blocks` 0 = one wave.
 int launch_wide(uint32_t id_bytes, bool slots, const GenArgs &a, unsigned long long *ticket,
                 uint32_t blocks, cudaStream_t s);
