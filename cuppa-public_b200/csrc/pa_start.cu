@@ -233,6 +233,7 @@ __global__ void __launch_bounds__(kThreads, MinBlocks) start_kernel(const StartA
     __shared__ unsigned long long s_seg[kThreads / 32][3];
     const uint32_t warp = threadIdx.x >> 5;
     GenArgs &a = s_args[warp];
+    cudaGridDependencySynchronize();
     if ((threadIdx.x & 31u) == 0) {
         s_seg[warp][0] = 1;   // empty segment
         s_seg[warp][1] = 0;
@@ -424,8 +425,18 @@ int launch_start_t(const StartArgs &b, uint32_t blocks, cudaStream_t s)
         if (need < g) g = need > 0 ? need : 1;
         blocks = (uint32_t)g;
     }
-    kern<<<blocks, kThreads, 0, s>>>(b);
-    const cudaError_t e = cudaGetLastError();
+    // launched while the kernel before it (the control block's and the fill's, of a
+    // small graph) still runs; start_kernel waits for its end
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(blocks);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    const cudaError_t e = cudaLaunchKernelEx(&cfg, kern, b);
     return e == cudaSuccess ? PA_OK : set_cuda_error(e);
 }
 

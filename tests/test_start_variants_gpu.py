@@ -63,3 +63,27 @@ def test_batch_in_the_scratch_of_coarse_levels(pa, cuda_ok):
         assert b.finish().status == 0
         assert all(torch.equal(b.graph(i), w) for i, w in enumerate(want))
     assert least is not None and least < full
+
+
+@pytest.mark.parametrize("layout", [0, 1])
+@pytest.mark.parametrize("bits", [32, 64])
+def test_one_launch_set_up(pa, cuda_ok, bits, layout):
+    """The control block, the claim counters and the region around a small graph's
+    edges: seed edges of odd counts (ragged region ends), a scratch and a buffer full of
+    other bytes, two generations in a row on one stream, sizes around the largest
+    region that is filled by the same launch (32 MB)."""
+    import torch
+    slot = (1 if layout else 2) * bits // 8
+    for n, d in [(50, 1), (1000, 3), (1001, 5), (3000, 40),
+                 ((32 << 20) // slot // 4 + 5, 4), ((32 << 20) // slot // 4 + 6, 4)]:
+        prm = pa.make_params(n, d, 0.5, seed=n, id_bits=bits, layout=layout)
+        G = orc.generate(n, d, 0.5, n, orc.SEED_CLIQUE)
+        want = G[d + 1:] if layout else orc.pairs_slot_order(G, orc.SEED_CLIQUE)
+        edges, scratch = pa.alloc_buffers(prm)
+        for byte in (0, 7):
+            edges.fill_(byte)
+            scratch.fill_(byte)
+            pa.generate_into(prm, edges, scratch)
+            pa.generate_into(prm, edges, scratch)
+            assert pa.finish(scratch).status == 0
+            assert (edges.cpu().numpy().astype(np.int64) == want).all()
