@@ -36,6 +36,16 @@ namespace pa {
 namespace {
 
 constexpr uint32_t kFull = 0xffffffffu;
+
+// First in every kernel of the build: let the next kernel's blocks come up (it
+// waits in turn, and starts only once every block of this one has), and wait for the
+// kernel before to have ended.
+__device__ __forceinline__ void follow()
+{
+    cudaTriggerProgrammaticLaunchCompletion();
+    cudaGridDependencySynchronize();
+}
+
 // ---------------------------------------------------------------------------
 // Seed rows' out parts for the path of d > 32 (rows_kernel writes them for
 // d <= 32; csr_out_wide writes the generated rows): the seed rows' out-edges go
@@ -125,6 +135,7 @@ __global__ void __launch_bounds__(kRadixThreads) radix_hist_all_kernel(const Id 
                                                                        uint32_t *err)
 {
     constexpr uint32_t NB = 1u << DB, MASK = NB - 1;
+    follow();
     __shared__ uint32_t cnt[kMaxPasses * NB];
     for (uint32_t b = threadIdx.x; b < kMaxPasses * NB; b += kRadixThreads) cnt[b] = 0;
     __syncthreads();
@@ -226,6 +237,7 @@ __global__ void __launch_bounds__(kRadixThreads, 2) radix_pass_kernel(
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31u;
     const uint32_t lt = lanemask_lt();
     const bool owner = tid * DPT < NB;
+    follow();
     if (tid == 0) S.tile = atomicAdd(tile_ctr, 1ull);
     for (uint32_t b = lane; b < NB; b += 32) S.word[warp][b] = make_uint2(0u, 0u);
     __syncthreads();
@@ -484,6 +496,7 @@ __global__ void __launch_bounds__(256) rowptr_kernel(const unsigned long long *i
                                                      uint32_t seed_mode, uint32_t span,
                                                      int64_t *rowptr)
 {
+    follow();
     __shared__ uint32_t s_key[256 / 32][kRowSpan];
     const uint32_t lane = threadIdx.x & 31u;
     uint32_t *key = s_key[threadIdx.x >> 5];
@@ -633,6 +646,7 @@ __global__ void __launch_bounds__(256) rows_kernel(const Id *E, const unsigned l
     const bool used = lane < G * d;
     const uint64_t step = warps * kRowsChunk;
     const uint64_t limit = heavy_limit(n_items, warps, d);
+    follow();
     // rowptr of each chunk's rows, and of the row after it, is loaded one chunk
     // ahead
     int64_t rp_next = 0, re_next = 0;
@@ -753,6 +767,7 @@ __global__ void __launch_bounds__(256) heavy_in_kernel(const unsigned long long 
                                                        const unsigned long long *ctr)
 {
     constexpr uint32_t PL = kPiece / 32;   // items per lane per piece
+    follow();
     const uint32_t lane = threadIdx.x & 31u;
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     const uint64_t w0 = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -812,6 +827,25 @@ int grid_for(uint64_t items, uint32_t threads, uint32_t per_sm = 8)
     uint64_t want = (items + threads - 1) / threads;
     const uint64_t cap = (uint64_t)sms * per_sm;
     return (int)(want == 0 ? 1 : (want > cap ? cap : want));
+}
+
+// Launch a kernel of the build while the one before it still runs: it waits for
+// that one's end itself (follow()), so its launch costs no time of its own.
+template <typename... P, typename... A>
+cudaError_t launch(void (*kern)(P...), uint64_t grid, uint32_t threads, size_t smem, cudaStream_t s,
+                   A... args)
+{
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)grid);
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = s;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kern, static_cast<P>(args)...);
 }
 
 struct CsrLayout {
@@ -903,13 +937,11 @@ int radix_sort(const Id *E, uint64_t m, uint64_t n, uint32_t passes, unsigned lo
     // four 512-thread blocks per SM (24 registers, 8 KB of counters each): at
     // n = 10^8, d = 16 the kernel took 8.44 ms with two blocks per SM, 5.96 ms
     // with four
-    radix_hist_all_kernel<Id, DB><<<grid_for(m / 4 + 1, kRadixThreads, 4), kRadixThreads, 0, s>>>(
-        E, m, n, passes, buf(0), hist, base, ctr + kMaxPasses + 1, err);
-    const unsigned tiles = (unsigned)r_tiles;
-    for (uint32_t q = 0; q < passes; ++q)
-        radix_pass_kernel<DB, R><<<tiles, kRadixThreads, smem, s>>>(
-            buf(q), buf(q + 1), m, DB * q, base + q * NB, status, q + 1, ctr + q, 2000000000ull, err);
-    e = cudaGetLastError();
+    e = launch(radix_hist_all_kernel<Id, DB>, grid_for(m / 4 + 1, kRadixThreads, 4), kRadixThreads, 0,
+               s, E, m, n, passes, buf(0), hist, base, ctr + kMaxPasses + 1, err);
+    for (uint32_t q = 0; q < passes && e == cudaSuccess; ++q)
+        e = launch(radix_pass_kernel<DB, R>, r_tiles, kRadixThreads, smem, s, buf(q), buf(q + 1), m,
+                   DB * q, base + q * NB, status, q + 1, ctr + q, 2000000000ull, err);
     return e == cudaSuccess ? PA_OK : set_cuda_error(e);
 }
 
@@ -974,14 +1006,17 @@ int csr_enqueue_t(const pa_params *prm, const GenPlan &p, const Id *E, int64_t *
         // the end of a graph, where few rows have in-edges, writes hundreds)
         uint32_t span = kRowSpan;
         while (span > 32 && m < (uint64_t)span * 148 * 64) span /= 2;
-        rowptr_kernel<<<grid_for(m / span + 1, 256 / 32), 256, 0, s>>>(A, m, n, d, p.seed_edges,
-                                                                       seed_mode, span, rowptr);
+        e = launch(rowptr_kernel, grid_for(m / span + 1, 256 / 32), 256, 0, s, A, m, n, d, p.seed_edges,
+                   seed_mode, span, rowptr);
         const int grid = grid_for(n / kRowsChunk + 1, 256 / 32);
-        rows_kernel<Id><<<grid, 256, 0, s>>>(E, A, m, rowptr, col, n, d, p.seed_edges, seed_mode,
-                                             col_len, heavy, pref, L.heavy_cap, lists);
+        if (e == cudaSuccess)
+            e = launch(rows_kernel<Id>, grid, 256, 0, s, E, A, m, rowptr, col, n, d, p.seed_edges,
+                       seed_mode, col_len, heavy, pref, L.heavy_cap, lists);
         // one warp per piece at least; at most m / kPiece + (listed chunks) pieces
-        heavy_in_kernel<Id><<<grid_for(m / kPiece + 1, 256 / 32), 256, 0, s>>>(
-            A, m, rowptr, col, n, d, p.seed_edges, seed_mode, col_len, heavy, pref, L.heavy_cap, lists);
+        if (e == cudaSuccess)
+            e = launch(heavy_in_kernel<Id>, grid_for(m / kPiece + 1, 256 / 32), 256, 0, s, A, m, rowptr,
+                       col, n, d, p.seed_edges, seed_mode, col_len, heavy, pref, L.heavy_cap, lists);
+        return e == cudaSuccess ? PA_OK : set_cuda_error(e);
     }
     e = cudaGetLastError();
     return e == cudaSuccess ? PA_OK : set_cuda_error(e);
