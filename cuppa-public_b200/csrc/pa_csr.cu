@@ -479,22 +479,28 @@ __global__ void in_sorted_kernel(const unsigned long long *items, uint64_t n_ite
 
 // rowptr alone (the row writer's input): rowptr[x] = outprefix(x) + the first
 // position k in [0, n_items] whose key is >= x (key(n_items) = n; keys >= n,
-// only after an input error, count as n).  A warp takes `span` (32 .. 256, a power
-// of two) consecutive positions and writes rows (key(k0 - 1), key(k0 + span - 1)],
-// one per lane, each from a binary search over the positions' keys, so a run of
-// rows without in-edges costs one coalesced store per row.  Issue-bound, so the
-// search depends on how many rows there are: up to kFewRows, over the whole span
-// in shared memory (one or two steps of 32 rows); more, by shuffles within the 32
-// positions that hold them (five steps instead of eight, no bank conflicts).
-// n = 2.5 * 10^7, d = 16: 1.25 ms by shuffles alone, now 0.75; n = 2^27, d = 4, p = 0.1,
-// CSR: 20.3 ms by shuffles alone, 22.5 in shared memory alone, now 20.4.
+// only after an input error, count as n).
+//
+// Rows and sorted items form one sequence, row x before the items of key >= x, and a
+// warp takes an even share of it, a row weighing kRowWeight items (its search; with
+// equal weights n = 2.5 * 10^7, d = 16 takes 0.13 ms longer): rows [x0, x1) and the items [k0, k1) among them,
+// found by two 16-way searches side by side.  (Shares of equal items only leave the
+// rows of a graph's end, where an item stands for fifty rows, to a few warps: n =
+// 3 * 10^6, d = 9, p = 0.2: 162 us, now 58.)  It goes through its items 256 at a time and
+// writes the rows up to the last one's key, one per lane, each from a binary search over
+// the keys.  Issue-bound, so the search depends on how many rows there are: up to
+// kFewRows, over the 256 positions in shared memory (one or two steps of 32 rows);
+// more, by shuffles within the 32 positions that hold them (five steps instead of
+// eight, no bank conflicts): n = 2.5 * 10^7, d = 16: 1.25 ms by shuffles alone, now 0.72; n =
+// 2^27, d = 4, p = 0.1, the whole CSR: 20.3 ms by shuffles alone, 22.5 in shared memory
+// alone, now 18.3.
+constexpr uint64_t kRowWeight = 4;
 constexpr uint32_t kFewRows = 64;
 constexpr uint32_t kRowSpan = 256;
 
 __global__ void __launch_bounds__(256) rowptr_kernel(const unsigned long long *items, uint64_t n_items,
                                                      uint64_t n, uint32_t d, uint64_t seed_edges,
-                                                     uint32_t seed_mode, uint32_t span,
-                                                     int64_t *rowptr)
+                                                     uint32_t seed_mode, int64_t *rowptr)
 {
     follow();
     __shared__ uint32_t s_key[256 / 32][kRowSpan];
@@ -502,42 +508,63 @@ __global__ void __launch_bounds__(256) rowptr_kernel(const unsigned long long *i
     uint32_t *key = s_key[threadIdx.x >> 5];
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     const uint64_t w0 = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const uint64_t positions = n_items + 1;
-    // keys, rows and the search in 32 bits (n < 2^32)
-    const uint32_t n32 = (uint32_t)n;
-    for (uint64_t c0 = w0 * span; c0 < positions; c0 += warps * span) {
-        // the first row not yet written: rows up to key(c0 - 1) belong to the
-        // warp holding position c0 - 1
-        uint64_t nxt = c0 == 0 ? 0 : min(items[c0 - 1] >> 32, (unsigned long long)n) + 1;
+    const uint64_t total = n_items + kRowWeight * (n + 1), share = (total + warps - 1) / warps;
+    const uint64_t d0 = min(w0 * share, total), d1 = min(d0 + share, total);
+    if (d0 == d1) return;
+    auto key_at = [&](uint64_t k) { return min(items[k] >> 32, (unsigned long long)n); };
+    uint64_t nxt, x1, k0, k1;
+    {
+        // lanes 0-15: the rows within weight d0 of the sequence, lanes 16-31: within d1;
+        // the largest x whose last row, x - 1, comes before the item then next
+        const uint64_t D = lane < 16 ? d0 : d1;
+        uint64_t lo = D > n_items ? (D - n_items) / kRowWeight : 0, hi = min(D / kRowWeight, n + 1);
+        while (__any_sync(kFull, lo < hi)) {
+            const uint64_t step = (hi - lo + 15) / 16;
+            const uint64_t x = min(lo + ((lane & 15u) + 1) * step, hi), k = D - kRowWeight * x;
+            const bool p = lo == hi || k >= n_items || key_at(k) + 1 >= x;
+            const uint32_t t = __popc((__ballot_sync(kFull, p) >> (lane & 16u)) & 0xffffu);
+            if (lo < hi) {
+                if (t < 16) hi = min(lo + (t + 1) * step, hi) - 1;
+                lo = min(lo + t * step, hi);
+            }
+        }
+        // and the items before row x: a row's weight may reach into them
+        uint64_t k = min(D - kRowWeight * lo, n_items);
+        while (k > 0 && key_at(k - 1) >= lo) --k;
+        nxt = __shfl_sync(kFull, lo, 0);
+        x1 = __shfl_sync(kFull, lo, 16);
+        k0 = __shfl_sync(kFull, k, 0);
+        k1 = __shfl_sync(kFull, k, 16);
+    }
+    for (uint64_t c0 = k0; nxt < x1; c0 += kRowSpan) {
+        // keys in 32 bits (n < 2^32); position k1 closes the share's rows
         uint32_t v[kRowSpan / 32];
 #pragma unroll
         for (uint32_t q = 0; q < kRowSpan / 32; ++q) {
             const uint64_t k = c0 + q * 32 + lane;
-            v[q] = n32;
-            if (q * 32 < span && k < n_items)
-                v[q] = (uint32_t)min(items[k] >> 32, (unsigned long long)n);
+            v[q] = (uint32_t)(x1 - 1);
+            if (k < k1) v[q] = (uint32_t)key_at(k);
         }
         __syncwarp();
 #pragma unroll
-        for (uint32_t q = 0; q < kRowSpan / 32; ++q)
-            if (q * 32 < span) key[q * 32 + lane] = v[q];
+        for (uint32_t q = 0; q < kRowSpan / 32; ++q) key[q * 32 + lane] = v[q];
         __syncwarp();
-        const uint32_t last = key[span - 1];
+        const uint32_t last = key[kRowSpan - 1];
         if (last <= nxt + kFewRows) {
             for (uint64_t x0 = nxt; x0 <= last; x0 += 32) {
                 const uint64_t x = x0 + lane;
                 if (x <= last) {
                     uint32_t lo = 0;   // positions of the span whose key is below x
-                    for (uint32_t step = span / 2; step > 0; step >>= 1)
+                    for (uint32_t step = kRowSpan / 2; step > 0; step >>= 1)
                         if (key[lo + step - 1] < (uint32_t)x) lo += step;
                     rowptr[x] = (int64_t)(outprefix(x, d, seed_edges, seed_mode) + c0 + lo);
                 }
             }
+            if ((uint64_t)last + 1 > nxt) nxt = (uint64_t)last + 1;
             continue;
         }
 #pragma unroll
         for (uint32_t q = 0; q < kRowSpan / 32; ++q) {
-            if (q * 32 >= span) break;   // warp-uniform
             const uint32_t last_q = __shfl_sync(kFull, v[q], 31);
             for (uint64_t x0 = nxt; x0 <= last_q; x0 += 32) {
                 const uint64_t x = x0 + lane;
@@ -1002,12 +1029,9 @@ int csr_enqueue_t(const pa_params *prm, const GenPlan &p, const Id *E, int64_t *
         unsigned long long *lists = (unsigned long long *)(scratch + L.ctr_off) + kMaxPasses;
         unsigned long long *heavy = (unsigned long long *)(scratch + L.heavy_off);
         unsigned long long *pref = (unsigned long long *)(scratch + L.pref_off);
-        // fewer positions a warp where 256 would leave SMs without work (a warp at
-        // the end of a graph, where few rows have in-edges, writes hundreds)
-        uint32_t span = kRowSpan;
-        while (span > 32 && m < (uint64_t)span * 148 * 64) span /= 2;
-        e = launch(rowptr_kernel, grid_for(m / span + 1, 256 / 32), 256, 0, s, A, m, n, d, p.seed_edges,
-                   seed_mode, span, rowptr);
+        // one share of the rows and items a warp, 128 of them at least
+        e = launch(rowptr_kernel, grid_for((m + n) / 128 + 1, 256 / 32), 256, 0, s, A, m, n, d,
+                   p.seed_edges, seed_mode, rowptr);
         const int grid = grid_for(n / kRowsChunk + 1, 256 / 32);
         if (e == cudaSuccess)
             e = launch(rows_kernel<Id>, grid, 256, 0, s, E, A, m, rowptr, col, n, d, p.seed_edges,
