@@ -99,12 +99,32 @@ __device__ __forceinline__ void classify_start(Slot<uint32_t> &s, const DrawT<ui
     }
 }
 
+// The lower lanes of this lane's node whose key equals this lane's.  Latency: the
+// launch is bound by the rounds of its chains, where up to three shuffles answer
+// sooner than a match over 32 distinct keys (n = 10^5, d = 4: 51.2 -> 46.4 us); they
+// take more instructions, which bind larger graphs (n = 2^24, p = 0: 3.83 against
+// 4.58 ms with shuffles).
+template <bool Latency>
+__device__ __forceinline__ uint32_t lower_equal(uint32_t key, const Lane &L, uint32_t d)
+{
+    if (Latency && d <= 4) {
+        uint32_t low = 0;
+#pragma unroll
+        for (uint32_t j = 1; j < 4; ++j) {
+            const uint32_t o = __shfl_up_sync(kFull, key, j);
+            if (L.slot >= j && o == key) low |= (1u << L.lane) >> j;
+        }
+        return L.used ? low : 0u;
+    }
+    return __match_any_sync(kFull, key) & L.lt & L.gmask;
+}
+
 // Resolve the P warp passes of one start tile together; every slot is
 // stored as soon as it is final.  Copy sources in the lane's own pass come from
 // the source lane by shuffle; sources in an earlier pass of the tile are polled
 // in memory like any other.  Returns false when the warp must stop (wait limit,
 // or another warp failed).
-template <typename Id, bool Slots, int P>
+template <typename Id, bool Slots, int P, bool Latency>
 __device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[P], const GenArgs &a,
                                               Id *E, uint32_t tb, bool withhold, const Lane &L,
                                               uint32_t &n_retry, uint32_t &n_wait,
@@ -150,8 +170,9 @@ __device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[P], const GenA
             dirty &= ~(1u << j);
             const bool known = active && meta_st(s[j].meta) == ST_KNOWN;
             // node values are < 2^31: the lane-unique keys of unknown lanes never collide
-            const uint32_t eq = __match_any_sync(kFull, known ? s[j].val : (0xffffffe0u | L.lane));
-            const bool bad = active && (!known || (eq & L.lt & L.gmask) != 0u);
+            const uint32_t low =
+                lower_equal<Latency>(known ? s[j].val : (0xffffffe0u | L.lane), L, d);
+            const bool bad = active && (!known || low != 0u);
             const uint32_t badm = __ballot_sync(kFull, bad);
             const bool fin = active && (badm & L.gmask & L.le) == 0u;
             if (fin && !((stored >> j) & 1u)) {
@@ -179,7 +200,7 @@ __device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[P], const GenA
             }
 
             // a candidate equal to a final lower slot of the node is rejected
-            if (known && !fin && (eq & L.lt & L.gmask & finm) != 0u) {
+            if (known && !fin && (low & finm) != 0u) {
                 const uint32_t r = meta_r(s[j].meta) + 1u;
                 classify_start<Id, Slots>(s[j], draw<uint32_t>(u, L.slot, r, a), r, a, E, pbase,
                                           n_pend);
@@ -360,8 +381,9 @@ __global__ void __launch_bounds__(kThreads, MinBlocks) start_kernel(const StartA
                     }
                 }
         }
-        ok = resolve_start<Id, Slots, P>(s, a, E, tb, a.withhold_first && t == 0, L, n_retry, n_wait,
-                                         n_pend, n_poll);
+        constexpr bool kLatency = P == 1 && MinBlocks == kStartMinBlocksMid;
+        ok = resolve_start<Id, Slots, P, kLatency>(s, a, E, tb, a.withhold_first && t == 0, L, n_retry,
+                                                   n_wait, n_pend, n_poll);
     }
 
 #pragma unroll
