@@ -127,8 +127,9 @@ __device__ __forceinline__ uint32_t lower_equal(uint32_t key, const Lane &L, uin
 template <typename Id, bool Slots, int P, bool Latency>
 __device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[P], const GenArgs &a,
                                               Id *E, uint32_t tb, bool withhold, const Lane &L,
-                                              uint32_t &n_retry, uint32_t &n_wait,
-                                              uint32_t &n_pend, uint32_t &n_poll)
+                                              uint32_t done, uint32_t &n_retry,
+                                              uint32_t &n_wait, uint32_t &n_pend,
+                                              uint32_t &n_poll)
 {
     const uint32_t d = a.d, G = a.groups;
     // this lane's slot of pass 0: a pair (PAIRS) or an id (SLOTS, seed_edges = 0)
@@ -141,9 +142,8 @@ __device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[P], const GenA
     const uint32_t max_sleep = min(a.max_sleep_ns, 512u);
     uint64_t spin_t0 = 0;
     uint32_t sleep_ns = 32;
-    // bit j: every active slot of pass j is final and stored (warp-uniform); a
-    // finished pass costs no more match or ballot while the others wait
-    uint32_t done = 0;
+    // done, bit j: every active slot of pass j is final and stored (warp-uniform);
+    // a finished pass costs no more match or ballot while the others wait
     // bit j: this lane's slot of pass j changed after the pass's last match; a
     // pass in which no lane changed would match and vote exactly as before, so
     // only its pending reads are polled (one vote per pass and round)
@@ -234,6 +234,58 @@ __device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[P], const GenA
             sleep_ns = 32;
         }
     }
+}
+
+// Store the passes of a tile that are settled as drawn: every slot known, no value
+// twice in a node.  Nearly all are, late in a large graph, and the rounds of
+// resolve_start, made for slots that wait, take several times the instructions
+// and a match each, which bound the launch where copies are few or in L2 (85 % of
+// the match unit, 65 % of the issue slots at n = 2^24, d = 4, p = 1).  Up to d = 8 equal
+// values are looked for by d - 1 shuffles.  Returns the stored passes.
+// n = 2^24, d = 4: p = 1 667 -> 492 us, p = 0.5 851 -> 805; n = 10^7 536 -> 494; n = 2^28,
+// p = 0.9 12.6 -> 10.3 ms; p = 0.5 there, bound by the copies' 128-byte lines, 16.2.
+template <typename Id, bool Slots, int P>
+__device__ __forceinline__ uint32_t store_settled(const Slot<uint32_t> (&s)[P], const GenArgs &a,
+                                                  Id *E, uint32_t tb, bool withhold, const Lane &L)
+{
+    const uint32_t d = a.d, pd = a.groups * d;
+    const uint64_t e_lane = a.seed_edges + (uint64_t)(tb - (uint32_t)a.u_first) * d + L.lane;
+    Id *to = Slots ? E + e_lane : E + 2 * e_lane;
+    uint32_t done = 0;
+#pragma unroll
+    for (int j = 0; j < P; ++j) {
+        const uint32_t u = tb + j * a.groups + L.g;
+        const bool active = L.used && u < a.start_end;
+        const uint32_t x = s[j].val;
+        Id *const at = to;
+        to += Slots ? pd : 2 * pd;
+        if (!__all_sync(kFull, !active || meta_st(s[j].meta) == ST_KNOWN)) continue;
+        bool dup = false;
+        if (d <= 4) {
+#pragma unroll
+            for (uint32_t q = 1; q < 4; ++q) {
+                const uint32_t o = __shfl_up_sync(kFull, x, q);
+                dup |= L.slot >= q && o == x;
+            }
+        } else if (d <= 8) {
+#pragma unroll
+            for (uint32_t q = 1; q < 8; ++q) {
+                const uint32_t o = __shfl_up_sync(kFull, x, q);
+                dup |= L.slot >= q && o == x;
+            }
+        } else {
+            // node values are < 2^31: the keys of other lanes never collide
+            const uint32_t eq = __match_any_sync(kFull, active ? x : (0xffffffe0u | L.lane));
+            dup = (eq & L.lt & L.gmask) != 0u;
+        }
+        if (__any_sync(kFull, active && dup)) continue;
+        if (active && !withhold) {
+            if constexpr (Slots) st_relaxed_id(at, x);
+            else st_relaxed_pair(at, u, x);
+        }
+        done |= 1u << j;
+    }
+    return done;
 }
 
 __device__ __forceinline__ void set_lane(Lane &L, const GenArgs &a)
@@ -382,8 +434,11 @@ __global__ void __launch_bounds__(kThreads, MinBlocks) start_kernel(const StartA
                 }
         }
         constexpr bool kLatency = P == 1 && MinBlocks == kStartMinBlocksMid;
-        ok = resolve_start<Id, Slots, P, kLatency>(s, a, E, tb, a.withhold_first && t == 0, L, n_retry,
-                                                   n_wait, n_pend, n_poll);
+        const bool withhold = a.withhold_first && t == 0;
+        const uint32_t done = store_settled<Id, Slots, P>(s, a, E, tb, withhold, L);
+        if (done != (1u << P) - 1u)
+            ok = resolve_start<Id, Slots, P, kLatency>(s, a, E, tb, withhold, L, done, n_retry, n_wait,
+                                                       n_pend, n_poll);
     }
 
 #pragma unroll
