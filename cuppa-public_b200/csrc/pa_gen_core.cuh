@@ -25,6 +25,7 @@ constexpr uint32_t kStartMinBlocksMid = 4;
 constexpr uint32_t kStartMinBlocksMany = 6;
 struct StartVariant {
     uint32_t min_blocks, passes;
+    bool hop = false;   // launches of growing node ranges, copies drawn again (pa_start.cu)
 };
 
 // The variant for one graph (start region nodes, chance of a direct pick).
@@ -49,6 +50,22 @@ inline StartVariant start_variant(uint64_t start_nodes, double p)
     if (p == 0.0 || (start_nodes < (1ull << 22) && p < 0.75)) return {kStartMinBlocksMany, 1};
     if (start_nodes <= (1ull << 24) && p < 0.75) return {kStartMinBlocks, 2};
     return {p < 0.95 ? kStartMinBlocksMid : kStartMinBlocks, (uint32_t)kStartPasses};
+}
+
+// Whether a graph with a start region of `bytes` is generated in hop launches (see
+// start_kernel): where most of its copies read DRAM and are what binds it, and few
+// slots are ever rejected.  Without -> with, ms (64-bit ids, d = 4 unless given):
+//  * n = 2^28, p = 0.5 15.82 -> 13.92, 0.4 18.36 -> 16.60, 0.6 14.12 -> 13.30; with fewer
+//    copies the draws cost more than the reads (0.7 11.69 -> 12.35), with more of
+//    them most are of copies (0.25 20.94 -> 20.44);
+//  * 2.1 GB, n = 2^25: 1.97 -> 1.86; 4.3 GB 3.90 -> 3.56, d = 8 4.03 -> 3.68; SLOTS 2.1 GB
+//    3.18 -> 3.05; 32-bit ids 8.6 GB 13.42 -> 12.26, d = 32 13.68 -> 12.81; below, the
+//    second-level cache answers more of the reads (1.6 GB, d = 5: 1.47 -> 1.50; 1 GB,
+//    p = 0.6: 1.22 -> 1.37).
+constexpr uint64_t kHopMinBytes = 2000000000ull;
+inline bool start_hops(uint64_t bytes, double p)
+{
+    return bytes >= kHopMinBytes && p >= 0.4 && p <= 0.6;
 }
 
 // The variant for a batch of graphs with `slots` slots: chains of a small batch
@@ -503,6 +520,15 @@ __device__ __forceinline__ void map_unit_seg(const LevelTables &tab, uint32_t co
 // addresses instead of one).
 constexpr uint32_t kStartCounters = kThreads / 32;
 
+// Hop launches (start_kernel): the filter has 2^kHopLog2 bits, the first launch
+// kHopFirstNodes nodes and each later one as many as all before it (half or a quarter
+// as many: no faster); nodes are below 2^31, so kHopMaxLaunches is never reached.
+// Each launch has claim counters of its own.
+constexpr uint32_t kHopLog2 = 17;
+constexpr uint64_t kHopFilterBytes = 1ull << (kHopLog2 - 3);
+constexpr uint64_t kHopFirstNodes = 1ull << 21;
+constexpr uint32_t kHopMaxLaunches = 16;
+
 // Start kernel (pa_start.cu): start tiles of one graph (count == 1, arguments in
 // `one`) or of `count` graphs in level order (arguments in `inst`).
 struct StartArgs {
@@ -511,7 +537,9 @@ struct StartArgs {
     LevelTables tab;
     uint32_t count;
     uint32_t write_seeds;          // also write every graph's seed edges
-    unsigned long long t_end;      // start tiles of the launch
+    unsigned long long t_begin, t_end;   // start tiles of the launch
+    uint32_t *rejected;            // hop launches: the filter of rejected slots
+    uint32_t hop_end;              // and the end of the nodes of earlier launches
     unsigned long long *ticket;    // kStartCounters claim counters, 128 bytes apart (zero)
     GenCtl *ctl;                   // shared status and counters
 };

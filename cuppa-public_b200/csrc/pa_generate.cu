@@ -553,8 +553,14 @@ int launch_generate(const pa_params *prm, const GenPlan &plan, void *d_edges, vo
         sa.one = a;
         sa.count = 1;
         sa.write_seeds = 1;
-        const StartVariant variant =
-            start_variant(plan.u_split - plan.u_first, plan.model == PA_MODEL_BA ? 0.5 : prm->p);
+        const double p = plan.model == PA_MODEL_BA ? 0.5 : prm->p;
+        StartVariant variant = start_variant(plan.u_split - plan.u_first, p);
+        // the filter and the launches' counters lie where tile flags would, unused here
+        constexpr uint64_t hop_bytes = kHopFilterBytes + kHopMaxLaunches * kStartAreaBytes;
+        const uint64_t slot_bytes = (plan.slots ? 1u : 2u) * plan.id_bytes;
+        if (alone && kCtlBytes + hop_bytes <= plan.start_offset &&
+            start_hops((plan.u_split - plan.u_first) * prm->d * slot_bytes, p))
+            variant = {kStartMinBlocksMid, (uint32_t)kStartPasses, true};
         const uint64_t tile_nodes = (uint64_t)variant.passes * plan.groups;
         sa.t_end = (plan.u_split - plan.u_first + tile_nodes - 1) / tile_nodes;
         sa.ticket = reinterpret_cast<unsigned long long *>(reinterpret_cast<unsigned char *>(d_scratch) +
@@ -562,8 +568,25 @@ int launch_generate(const pa_params *prm, const GenPlan &plan, void *d_edges, vo
         sa.ctl = a.ctl;
         mrc = mark(1);
         if (mrc != PA_OK) return mrc;
-        const int rc = launch_start(plan.id_bytes, sa, blocks, stream, plan.slots, variant);
-        if (rc != PA_OK) return rc;
+        const unsigned long long tiles = sa.t_end;
+        if (variant.hop) {
+            unsigned char *spare = reinterpret_cast<unsigned char *>(d_scratch) + kCtlBytes;
+            e = cudaMemsetAsync(spare, 0, hop_bytes, stream);
+            if (e != cudaSuccess) return set_cuda_error(e);
+            sa.rejected = reinterpret_cast<uint32_t *>(spare);
+            sa.ticket = reinterpret_cast<unsigned long long *>(spare + kHopFilterBytes);
+            sa.t_end = std::min<unsigned long long>(tiles, kHopFirstNodes / tile_nodes);
+        }
+        for (uint32_t l = 1;; ++l) {
+            const int rc = launch_start(plan.id_bytes, sa, blocks, stream, plan.slots, variant);
+            if (rc != PA_OK) return rc;
+            if (sa.t_end == tiles) break;
+            sa.write_seeds = 0;
+            sa.t_begin = sa.t_end;
+            sa.t_end = l + 1 < kHopMaxLaunches ? std::min(tiles, 2 * sa.t_end) : tiles;
+            sa.hop_end = (uint32_t)(plan.u_first + sa.t_begin * tile_nodes);
+            sa.ticket += kStartAreaBytes / sizeof(*sa.ticket);
+        }
         if (plan.u_split >= prm->n) {
             mrc = mark(2);
             return mrc != PA_OK ? mrc : mark(3);

@@ -119,17 +119,24 @@ __device__ __forceinline__ uint32_t lower_equal(uint32_t key, const Lane &L, uin
     return __match_any_sync(kFull, key) & L.lt & L.gmask;
 }
 
+// The bit of slot (v, k) in the filter of rejected slots (start_kernel).
+__device__ __forceinline__ uint32_t hop_bit(uint32_t v, uint32_t k, uint32_t d)
+{
+    return ((v * d + k) * 0x9E3779B1u) >> (32u - kHopLog2);
+}
+
 // Resolve the P warp passes of one start tile together; every slot is
 // stored as soon as it is final.  Copy sources in the lane's own pass come from
 // the source lane by shuffle; sources in an earlier pass of the tile are polled
 // in memory like any other.  Returns false when the warp must stop (wait limit,
-// or another warp failed).
-template <typename Id, bool Slots, int P, bool Latency>
+// or another warp failed).  Hop: slots that end on a later draw than their first are
+// entered in the filter `rejected`.
+template <typename Id, bool Slots, int P, bool Latency, bool Hop>
 __device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[P], const GenArgs &a,
                                               Id *E, uint32_t tb, bool withhold, const Lane &L,
-                                              uint32_t done, uint32_t &n_retry,
-                                              uint32_t &n_wait, uint32_t &n_pend,
-                                              uint32_t &n_poll)
+                                              uint32_t done, uint32_t *rejected,
+                                              uint32_t &n_retry, uint32_t &n_wait,
+                                              uint32_t &n_pend, uint32_t &n_poll)
 {
     const uint32_t d = a.d, G = a.groups;
     // this lane's slot of pass 0: a pair (PAIRS) or an id (SLOTS, seed_edges = 0)
@@ -181,6 +188,10 @@ __device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[P], const GenA
                     else st_relaxed_pair(pair0 + 2 * (uint64_t)(j * G * d), u, s[j].val);
                 }
                 stored |= 1u << j;
+                if (Hop && meta_r(s[j].meta) != 0u) {
+                    const uint32_t h = hop_bit(u, L.slot, d);
+                    atomicOr(rejected + (h >> 5), 1u << (h & 31u));
+                }
             }
             const uint32_t finm = __ballot_sync(kFull, fin || !active);
             if (finm == kFull) {
@@ -243,7 +254,7 @@ __device__ __forceinline__ bool resolve_start(Slot<uint32_t> (&s)[P], const GenA
 // the match unit, 65 % of the issue slots at n = 2^24, d = 4, p = 1).  Up to d = 8 equal
 // values are looked for by d - 1 shuffles.  Returns the stored passes.
 // n = 2^24, d = 4: p = 1 667 -> 492 us, p = 0.5 851 -> 805; n = 10^7 536 -> 494; n = 2^28,
-// p = 0.9 12.6 -> 10.3 ms; p = 0.5 there, bound by the copies' 128-byte lines, 16.2.
+// p = 0.9 12.6 -> 10.3 ms.
 template <typename Id, bool Slots, int P>
 __device__ __forceinline__ uint32_t store_settled(const Slot<uint32_t> (&s)[P], const GenArgs &a,
                                                   Id *E, uint32_t tb, bool withhold, const Lane &L)
@@ -296,9 +307,21 @@ __device__ __forceinline__ void set_lane(Lane &L, const GenArgs &a)
     L.gmask = L.used ? (a.d == 32 ? kFull : (((1u << a.d) - 1u) << (L.g * a.d))) : 0u;
 }
 
-template <typename Id, bool Slots, uint32_t MinBlocks, int P>
+// Hop.  The copies of a large graph are bound by DRAM, which moves 128 bytes for a
+// slot's 4 to 16 (n = 2^28, d = 4, p = 0.5: 69 GB for half as many slots of 16).  But slot
+// (v, k) holds what its own first draw gave, unless that was rejected: was the draw
+// direct, its value is known without a read, and was it a copy, that one's slot is
+// read instead.  So such a graph is launched in growing ranges of nodes; every slot
+// that ends on a later draw leaves a hashed bit in a filter (false hits cost a read);
+// and copies of earlier launches' slots (below hop_end: final, their bits set) that
+// the filter, held in shared memory, does not hold are drawn again.  One draw of the
+// warp serves each lane's first such copy of the tile's four passes: draws take
+// instructions, which bind the launch next (a draw per copy of two passes 14.31 ms,
+// of all four 16.13, two draws as here 14.27, one 13.92; none 15.82).
+template <typename Id, bool Slots, uint32_t MinBlocks, int P, bool Hop>
 __global__ void __launch_bounds__(kThreads, MinBlocks) start_kernel(const StartArgs b)
 {
+    __shared__ uint32_t s_rejected[Hop ? kHopFilterBytes / 4 : 1];
     __shared__ GenArgs s_args[kThreads / 32];
     // per warp: the (level, graph) segment of its last claim, [lo, hi) and the
     // local unit of lo -- a warp's claims T, T + 8, ... mostly stay inside one,
@@ -312,6 +335,12 @@ __global__ void __launch_bounds__(kThreads, MinBlocks) start_kernel(const StartA
         s_seg[warp][1] = 0;
     }
     __syncwarp();
+    if constexpr (Hop) {
+        for (uint32_t i = threadIdx.x; i < kHopFilterBytes / 16; i += kThreads)
+            reinterpret_cast<uint4 *>(s_rejected)[i] =
+                reinterpret_cast<const uint4 *>(b.rejected)[i];
+        __syncthreads();
+    }
 
     Lane L;
     L.lane = threadIdx.x & 31u;
@@ -356,7 +385,7 @@ __global__ void __launch_bounds__(kThreads, MinBlocks) start_kernel(const StartA
         unsigned long long c = 0;
         if (L.lane == 0) c = atomicAdd(my_ticket, 1ull);
         c = __shfl_sync(kFull, c, 0);
-        const unsigned long long T = c * kStartCounters + warp;
+        const unsigned long long T = b.t_begin + c * kStartCounters + warp;
         if (T >= b.t_end) break;
         uint32_t i = 0;
         uint64_t t = T;
@@ -416,6 +445,25 @@ __global__ void __launch_bounds__(kThreads, MinBlocks) start_kernel(const StartA
                     place_start(s[j], draw<uint32_t>(u, L.slot, 0u, a), 0u, a, pbase))
                     reads |= 1u << j;
             }
+            if constexpr (Hop) {
+                uint32_t cand = 0;   // bit j: pass j's copy is of an earlier launch's slot
+#pragma unroll
+                for (int j = 0; j < P; ++j)
+                    if (((reads >> j) & 1u) && s[j].val < b.hop_end) cand |= 1u << j;
+                const uint32_t bit = cand & (0u - cand);
+                Slot<uint32_t> q = s[0];
+#pragma unroll
+                for (int j = 1; j < P; ++j)
+                    if (bit == 1u << j) q = s[j];
+                const uint32_t h = hop_bit(q.val, meta_k(q.meta), a.d);
+                const DrawT<uint32_t> dr = draw<uint32_t>(q.val, meta_k(q.meta), 0u, a);
+                if (bit != 0u && ((s_rejected[h >> 5] >> (h & 31u)) & 1u) == 0u) {
+                    if (!place_start(q, dr, 0u, a, b.hop_end)) reads ^= bit;
+#pragma unroll
+                    for (int j = 0; j < P; ++j)
+                        if (bit == 1u << j) s[j] = q;
+                }
+            }
 #pragma unroll
             for (int j = 0; j < P; ++j)
                 if ((reads >> j) & 1u)
@@ -437,8 +485,9 @@ __global__ void __launch_bounds__(kThreads, MinBlocks) start_kernel(const StartA
         const bool withhold = a.withhold_first && t == 0;
         const uint32_t done = store_settled<Id, Slots, P>(s, a, E, tb, withhold, L);
         if (done != (1u << P) - 1u)
-            ok = resolve_start<Id, Slots, P, kLatency>(s, a, E, tb, withhold, L, done, n_retry, n_wait,
-                                                       n_pend, n_poll);
+            ok = resolve_start<Id, Slots, P, kLatency, Hop>(s, a, E, tb, withhold, L, done,
+                                                            b.rejected, n_retry, n_wait,
+                                                            n_pend, n_poll);
     }
 
 #pragma unroll
@@ -485,10 +534,10 @@ __global__ void fill_start_kernel(const GenArgs *inst, uint32_t y0, uint32_t id_
         p[x] = ones;
 }
 
-template <typename Id, bool Slots, uint32_t MinBlocks, int P>
+template <typename Id, bool Slots, uint32_t MinBlocks, int P, bool Hop>
 int launch_start_t(const StartArgs &b, uint32_t blocks, cudaStream_t s)
 {
-    auto kern = start_kernel<Id, Slots, MinBlocks, P>;
+    auto kern = start_kernel<Id, Slots, MinBlocks, P, Hop>;
     if (blocks == 0) {
         int dev = 0, sms = 0, per_sm = 0;
         cudaError_t e = cudaGetDevice(&dev);
@@ -498,7 +547,7 @@ int launch_start_t(const StartArgs &b, uint32_t blocks, cudaStream_t s)
         if (e != cudaSuccess) return set_cuda_error(e);
         uint64_t g = (uint64_t)sms * (uint64_t)(per_sm > 0 ? per_sm : 1);
         // no more warps than start tiles (but one block at least, for the seed edges)
-        const uint64_t need = (b.t_end + kThreads / 32 - 1) / (kThreads / 32);
+        const uint64_t need = (b.t_end - b.t_begin + kThreads / 32 - 1) / (kThreads / 32);
         if (need < g) g = need > 0 ? need : 1;
         blocks = (uint32_t)g;
     }
@@ -519,15 +568,15 @@ int launch_start_t(const StartArgs &b, uint32_t blocks, cudaStream_t s)
 
 }  // namespace
 
-template <uint32_t MinBlocks, int P>
+template <uint32_t MinBlocks, int P, bool Hop = false>
 int launch_start_m(uint32_t id_bytes, const StartArgs &b, uint32_t blocks, cudaStream_t s,
                    bool slots)
 {
     if (slots)
-        return id_bytes == 8 ? launch_start_t<int64_t, true, MinBlocks, P>(b, blocks, s)
-                             : launch_start_t<int32_t, true, MinBlocks, P>(b, blocks, s);
-    return id_bytes == 8 ? launch_start_t<int64_t, false, MinBlocks, P>(b, blocks, s)
-                         : launch_start_t<int32_t, false, MinBlocks, P>(b, blocks, s);
+        return id_bytes == 8 ? launch_start_t<int64_t, true, MinBlocks, P, Hop>(b, blocks, s)
+                             : launch_start_t<int32_t, true, MinBlocks, P, Hop>(b, blocks, s);
+    return id_bytes == 8 ? launch_start_t<int64_t, false, MinBlocks, P, Hop>(b, blocks, s)
+                         : launch_start_t<int32_t, false, MinBlocks, P, Hop>(b, blocks, s);
 }
 
 int launch_start(uint32_t id_bytes, const StartArgs &b, uint32_t blocks, cudaStream_t s,
@@ -537,6 +586,8 @@ int launch_start(uint32_t id_bytes, const StartArgs &b, uint32_t blocks, cudaStr
         return v.min_blocks == kStartMinBlocksMany
                    ? launch_start_m<kStartMinBlocksMany, 1>(id_bytes, b, blocks, s, slots)
                    : launch_start_m<kStartMinBlocksMid, 1>(id_bytes, b, blocks, s, slots);
+    if (v.hop)
+        return launch_start_m<kStartMinBlocksMid, kStartPasses, true>(id_bytes, b, blocks, s, slots);
     if (v.passes == 2) return launch_start_m<kStartMinBlocks, 2>(id_bytes, b, blocks, s, slots);
     if (v.min_blocks == kStartMinBlocksMid)
         return launch_start_m<kStartMinBlocksMid, kStartPasses>(id_bytes, b, blocks, s, slots);
