@@ -28,26 +28,34 @@ struct StartVariant {
     bool hop = false;   // launches of growing node ranges, copies drawn again (pa_start.cu)
 };
 
-// The variant for one graph (start region nodes, chance of a direct pick).
+// The variant for one graph (start region nodes, d, chance of a direct pick).
 // Measured, one graph a call, against 40 warps with four passes throughout (us):
 //  * a graph below 2^20 nodes is bound by the latency of its dependency chains,
 //    and a step of a chain takes a round of the tile's loop, so tiles of one pass
 //    (n = 10^5, d = 4: 63 -> 53; d = 16: 211 -> 137; n = 10^4, p = 0: 268 -> 115), with
 //    no spills lengthening the round (48 warps: 61; 150; 122);
-//  * up to 2^22 nodes warps count as well (n = 3 * 10^6, d = 16: 833 -> 718; 820 at
-//    32 warps), unless few slots are copies and there is little to wait for
-//    (p = 1: 138 -> 165);
-//  * above, two, then four passes a tile, whose draws overlap and whose first reads
+//  * so is one below 2^23 slots (n = 1.1 * 10^6, d = 4, p = 0.5 112 with 48 warps, 101;
+//    n = 2 * 10^6, p = 0.3 168, 159);
+//  * up to 2^21 nodes, and to 2^22 if p < 0.25, warps count as well (n = 1.1 * 10^6, d = 32,
+//    p = 0.3 818; 855 with two passes, 856 at 32 warps; n = 3 * 10^6, d = 4, p = 0.1 275;
+//    294 with two passes), unless few slots are copies and there is little to wait
+//    for (p = 1: 138 -> 165);
+//  * above (n = 3 * 10^6, p = 0.5: d = 4 209 with 48 warps, 194 with two passes; d = 16 841
+//    and 699), two, then four passes a tile, whose draws overlap and whose first reads
 //    go out together (n = 5 * 10^6, d = 7, p = 0.3: 696 -> 600 with two passes at 40 warps;
 //    n = 2^24, d = 4: 978 -> 853; n = 2^28, 64-bit ids: 16,580 -> 15,850; one pass
 //    a tile: 1,085 and 20,800, bound by the claim counters); at p = 1, with no reads,
 //    the 40 warps stay ahead (n = 2^28: 11,424 against 11,740);
 //  * p = 0, every slot a copy and several retries per node, whose passes differ
 //    most in their number of rounds: one pass a tile (n = 2^24: 4,390 -> 3,840).
-inline StartVariant start_variant(uint64_t start_nodes, double p)
+inline StartVariant start_variant(uint64_t start_nodes, uint32_t d, double p)
 {
     if (start_nodes < (1ull << 20)) return {kStartMinBlocksMid, 1};
-    if (p == 0.0 || (start_nodes < (1ull << 22) && p < 0.75)) return {kStartMinBlocksMany, 1};
+    if (p == 0.0) return {kStartMinBlocksMany, 1};
+    if (start_nodes < (1ull << 22) && p < 0.75) {
+        if (start_nodes * d < (1ull << 23)) return {kStartMinBlocksMid, 1};
+        if (start_nodes < (1ull << 21) || p < 0.25) return {kStartMinBlocksMany, 1};
+    }
     if (start_nodes <= (1ull << 24) && p < 0.75) return {kStartMinBlocks, 2};
     return {p < 0.95 ? kStartMinBlocksMid : kStartMinBlocks, (uint32_t)kStartPasses};
 }

@@ -554,7 +554,7 @@ int launch_generate(const pa_params *prm, const GenPlan &plan, void *d_edges, vo
         sa.count = 1;
         sa.write_seeds = 1;
         const double p = plan.model == PA_MODEL_BA ? 0.5 : prm->p;
-        StartVariant variant = start_variant(plan.u_split - plan.u_first, p);
+        StartVariant variant = start_variant(plan.u_split - plan.u_first, prm->d, p);
         // the filter and the launches' counters lie where tile flags would, unused here
         constexpr uint64_t hop_bytes = kHopFilterBytes + kHopMaxLaunches * kStartAreaBytes;
         const uint64_t slot_bytes = (plan.slots ? 1u : 2u) * plan.id_bytes;

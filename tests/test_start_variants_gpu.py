@@ -28,6 +28,13 @@ def test_variants_match_oracle(pa, cuda_ok, n, d, p):
     assert (got.astype(np.int64) == want).all()
 
 
+@pytest.mark.parametrize("p", [0.1, 0.3])
+@pytest.mark.parametrize("n,d", [(2 ** 21 + 5 + x, 4) for x in (-1, 0)] + [(2 ** 21 + 6, 5)])
+def test_variants_by_slots(pa, cuda_ok, n, d, p):
+    """The lines at 2^23 slots, 2^21 nodes and p = 1/4."""
+    test_variants_match_oracle(pa, cuda_ok, n, d, p)
+
+
 def test_ba_above_the_lines(pa, cuda_ok):
     for n in (2 ** 20 + 9, 2 ** 22 + 9):
         prm = pa.make_params(n, 2, 0.0, seed=5, id_bits=64, seed_mode=pa.PA_SEED_STAR_REF,
