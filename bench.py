@@ -46,6 +46,7 @@ from __future__ import annotations
 
 import argparse
 import json
+import math
 import os
 import statistics
 import subprocess
@@ -510,7 +511,14 @@ def run_gpu(args, w):
             kernel, k_edges, kern_s = "start_kernel", start_edges, statistics.mean(start_ms) / 1e3
         achieved = k_edges * bpe / kern_s / 1e9
         traffic = load_traffic(args.workload)     # ncu DRAM bytes of one such launch
-        launches = (1 if u_split > w["d"] + 1 else 0) + (1 if gen_edges > 0 else 0)
+        # set-up kernel, start kernel (a launch per range of nodes, doubling from 2^21, in
+        # graphs that draw copied slots again), tile kernel
+        nodes = u_split - (w["d"] + 1)
+        p_eff = 0.5 if w.get("model", COPY) == BA else w["p"]
+        hops = (gen_edges <= 0 and 0.4 <= p_eff <= 0.6
+                and nodes * w["d"] * 2 * (w["id_bits"] // 8) >= 2_000_000_000)
+        launches = ((1 + (1 + math.ceil(math.log2(nodes / 2 ** 21)) if hops else 1)
+                     if nodes > 0 else 0) + (1 if gen_edges > 0 else 0))
         line = {
             "metric": w.get("metric", METRIC), "value": value, "unit": "edges/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps,
@@ -941,7 +949,7 @@ def measure_served(args, rate: float, seconds: float, outputs_name: str, world: 
         "express_sized": pcts(True), "bulk_sized": pcts(False),
         "all_ok": ok, "server_stats_rank0": st,
         "statuses_rank0": {str(c): statuses.count(c) for c in sorted(set(statuses))},
-        "gpu_launches": st["batches"] * 2 + (st["completed"] * 11 if outputs & pa.PA_OUT_CSR else 0),
+        "gpu_launches": st["batches"] * 2 + (st["completed"] * 6 if outputs & pa.PA_OUT_CSR else 0),
         "clocks": clk.summary(),
     }
     return fig, ok
