@@ -25,3 +25,31 @@ def test_hop_launches_match_tile_kernels(pa, cuda_ok, n, d, p, bits, slots, mode
         b = b[-(n - d - 1) * d:, 1].view(n - d - 1, d)
     assert torch.equal(a, b)
     assert sa.retries == sb.retries
+
+
+def test_hop_launches_captured_prefilled_and_on_few_blocks(pa, cuda_ok):
+    """The same graph from a replayed plan into dirty scratch, from a buffer filled
+    beforehand, and from grids of 3 and 500 blocks."""
+    import torch
+    kw = dict(seed=3, id_bits=64)
+    n, d, p = 2 ** 25 + 3, 4, 0.5
+    want, st = pa.generate(pa.make_params(n, d, p, **kw))
+    prm = pa.make_params(n, d, p, **kw)
+    edges, scratch = pa.alloc_buffers(prm)
+    scratch.fill_(0xab)
+    plan = pa.Plan(prm, edges, scratch)
+    for _ in range(2):
+        edges.zero_()
+        plan.launch()
+        assert pa.finish(scratch).status == 0
+        assert torch.equal(edges[: want.shape[0]], want)
+    plan.close()
+    for extra in (dict(flags=pa.PA_FLAG_PREFILLED), dict(blocks=3), dict(blocks=500)):
+        q = pa.make_params(n, d, p, **kw, **extra)
+        edges.zero_()
+        scratch.fill_(0xcd)
+        if "flags" in extra:
+            pa.fill(q, edges)
+        pa.generate_into(q, edges, scratch)
+        assert pa.finish(scratch).status == 0
+        assert torch.equal(edges[: want.shape[0]], want)
