@@ -1,35 +1,43 @@
 // pa_server.cu -- the request server: continuous batching of generation
 // requests under a device-memory budget.
 //
-// One control thread per server owns the server's CUDA streams and memory
-// pools on its device.  Client threads only touch host state (under the server
-// mutex): submit queues a request with the admission queue (pa_sched.cpp),
-// poll/wait read its state, release hands its buffer back.
+// Client threads only touch host state (under the server mutex): submit queues a
+// request with the admission queue (pa_sched.cpp), poll/wait read its state,
+// release hands its buffer back.
 //
 // Two lanes share the budget.  Requests of at most express_edges edges go to
-// the express lane, the rest to the bulk lane.  Each lane has one stream (the
-// express lane's at the device's highest stream priority), on which up to
-// max_inflight of its launches queue in order, and a memory pool of its own, so
-// that an allocation never waits for memory freed behind the other lane's
+// the express lane, the rest to the bulk lane.  Each lane has a control thread,
+// one stream (the express lane's at the device's highest stream priority), on which
+// up to max_inflight of its launches queue in order, and a memory pool of its own,
+// so that an allocation never waits for memory freed behind the other lane's
 // work.  Kernels are not preempted, but the block scheduler hands SMs that free
 // up to waiting blocks of higher-priority streams first: a small request that
-// arrives while a large batch runs starts at the batch's next kernel boundary
-// (a start kernel's tail, or between its CSR kernels) instead of after the
-// whole batch.
+// arrives while a large batch runs starts as the blocks of the kernel then running
+// end, instead of after the whole batch.
 //
-// The control thread loops, never waiting on the GPU:
-//   1. completions: for each in-flight launch whose event has fired, read the
+// A lane hands out the memory of a range of its own (DeviceRange), an eighth of the
+// budget for the express lane and the rest for the bulk lane: an allocation from a
+// pool that has become fragmented has the driver map memory, move it or wait
+// (measured: 6 ms a GB to grow a pool, 24 to 112 ms to close 2 GB holes, up to 1.6 s
+// under the served workload), with the control thread standing in the call.  The pool
+// is the last resort, when nothing that would give memory back is in flight.  Two
+// threads, because a stream's queue holds some thousand launches: the bulk lane's
+// thread waits when it is full.
+//
+// A control thread loops, never waiting on the GPU:
+//   1. completions: for each launch of the lane whose event has fired, read the
 //      device status it copied back, mark its requests done and return their
 //      generation scratch to the budget; retired launches (an error after part
 //      of a launch was queued) give their staging buffers back the same way;
 //   2. frees: buffers of released (or TTL-expired) results are freed on the
 //      stream that made them and their budget returned;
-//   3. admission: for each lane with room in flight, admit what fits the budget
+//   3. admission: with room in flight, admit what fits the budget
 //      and launch it as one batch per id width (the fill / start / tail launches
 //      of pa_batch.cu) -- requests that arrived while earlier batches ran make
-//      up the next; a group whose allocations fail (a fragmented pool) waits,
+//      up the next; a group whose allocations fail (a fragmented range) waits,
 //      admitted, for the next completion and is retried;
-//   4. sleep briefly (20 us with work in flight, else until woken).
+//   4. sleep briefly (20 us with work in flight, else until woken: by requests, and
+//      by budget that either lane gives back).
 // Memory per request: its edge buffer plus the generation scratch of its own
 // plan, which bounds its share of the batch scratch; with CSR outputs also its
 // rowptr, col and CSR scratch.  The CSR of every request of a batch is queued
@@ -45,11 +53,13 @@
 #include <deque>
 #include <mutex>
 #include <new>
+#include <system_error>
 #include <thread>
 #include <unordered_map>
 #include <vector>
 
 #include "pa_batch.h"
+#include "pa_range.h"
 
 namespace pa {
 namespace {
@@ -68,8 +78,7 @@ struct Request {
     uint64_t t_submit = 0, t_start = 0, t_done = 0;
     ReqState state = RQ_QUEUED;
     bool batchable = true;
-    uint32_t lane = 0;                 // kBulk or kExpress
-    cudaStream_t stream = nullptr;     // the stream that made (and frees) its buffers
+    uint32_t lane = 0;                 // kBulk or kExpress, which made (and frees) its buffers
 };
 
 constexpr uint32_t kBulk = 0, kExpress = 1, kLanes = 2;
@@ -86,16 +95,14 @@ struct Launch {
     Pinned buf;            // image; then the generation status word at status_off and
     uint64_t status_off = 0;   // one CSR status word per request after it
     cudaEvent_t done = nullptr;
-    cudaStream_t stream = nullptr;
 };
 
 // Staging of a launch that failed after part of it was queued: returned to the
 // pools once the work queued before the failure has run.
 struct Retired {
     cudaEvent_t done = nullptr;
-    cudaStream_t stream = nullptr;
     Pinned buf;
-    std::vector<void *> device;   // freed on `stream` when `done` fires
+    std::vector<void *> device;   // freed on the lane's stream when `done` fires
 };
 
 // What the control thread needs of an admitted request (copied under the lock).
@@ -105,12 +112,26 @@ struct Job {
     uint64_t edges_bytes, rowptr_bytes, col_bytes, csr_scratch;
 };
 
+// Work for a lane's control thread: free the buffer (if any), then return the
+// ticket's whole budget (if the ticket is not 0).
+struct Free {
+    uint64_t ticket;
+    void *ptr;
+};
+
+// A lane: its control thread's alone, but for to_free (under the server mutex).
 struct LaneState {
-    std::vector<cudaStream_t> streams;             // one stream: launches queue in order
-    cudaMemPool_t pool = nullptr;                  // the lane's own device memory
-    std::vector<Launch> inflight;                  // each on one of `streams`
+    cudaStream_t stream = nullptr;                 // launches queue in order
+    DeviceRange range;                             // the lane's share of the budget
+    cudaMemPool_t pool = nullptr;                  // memory beyond it
+    std::vector<Launch> inflight;
+    std::vector<Retired> retired;
+    std::vector<Pinned> pinned_free;
     std::deque<std::pair<std::vector<Job>, bool>> deferred;   // groups (batch?) waiting to
                                                                // be retried after a completion
+    uint64_t deferred_at = 0;                      // server's `gave` when they last were
+    std::vector<Free> to_free;
+    std::thread worker;
 };
 
 uint64_t scratch_reserve(const pa_params &prm, bool batchable)
@@ -132,26 +153,18 @@ struct pa_server {
     uint64_t express_edges = 0;
     std::mutex mu;
     std::condition_variable cv_work, cv_done;
-    std::thread worker;
     bool stop = false;
+    uint64_t events = 0;      // anything the control threads may be asleep to
+    uint64_t gave = 0;        // completions and frees: memory and budget given back
+    uint32_t active = 0;      // groups of both lanes being launched, in flight or retired
+    uint32_t running = 0;     // control threads
     pa_sched *sched = nullptr;
     std::unordered_map<uint64_t, Request> reqs;
-    // work for the control thread: free the buffer (if any) on the stream, then
-    // return the ticket's whole budget (if the ticket is not 0)
-    struct Free {
-        uint64_t ticket;
-        void *ptr;
-        cudaStream_t stream;
-    };
-    std::vector<Free> to_free;
     std::deque<std::pair<uint64_t, uint64_t>> done_order;  // t_done, ticket (TTL)
     uint64_t next_ticket = 1;
     std::chrono::steady_clock::time_point t0;
     pa_server_stats st{};
-    // control thread only
     LaneState lanes[kLanes];
-    std::vector<Retired> retired;
-    std::vector<Pinned> pinned_free;
 
     uint64_t now() const
     {
@@ -163,35 +176,46 @@ struct pa_server {
 
 namespace {
 
-Pinned get_pinned(pa_server *S, uint64_t bytes)
+constexpr uint64_t kPinnedBytes = 1ull << 20;   // a staging buffer's least size
+
+Pinned get_pinned(LaneState &LS, uint64_t bytes)
 {
-    for (size_t i = 0; i < S->pinned_free.size(); ++i)
-        if (S->pinned_free[i].cap >= bytes) {
-            Pinned b = S->pinned_free[i];
-            S->pinned_free.erase(S->pinned_free.begin() + (ptrdiff_t)i);
+    for (size_t i = 0; i < LS.pinned_free.size(); ++i)
+        if (LS.pinned_free[i].cap >= bytes) {
+            Pinned b = LS.pinned_free[i];
+            LS.pinned_free.erase(LS.pinned_free.begin() + (ptrdiff_t)i);
             return b;
         }
     Pinned b;
-    b.cap = std::max<uint64_t>(bytes, 1ull << 20);
+    b.cap = std::max<uint64_t>(bytes, kPinnedBytes);
     if (cudaMallocHost(&b.p, b.cap) != cudaSuccess) b = Pinned{};
     return b;
 }
 
+// Wake the control threads (lock held).
+void wake(pa_server *S)
+{
+    ++S->events;
+    S->cv_work.notify_all();
+}
+
 // Queue a request's buffers for freeing and its budget for return (lock held).
-// Buffers are freed in order on the stream that made them (the lane's stream,
-// whose pool owns them).
+// Buffers are freed in order on the stream that made them (the lane's, whose pool
+// owns them).
 void drop_buffers(pa_server *S, uint64_t tk, Request &r)
 {
+    std::vector<Free> &to_free = S->lanes[r.lane].to_free;
     for (void *b : {r.edges, (void *)r.rowptr, r.col})
-        if (b) S->to_free.push_back({0, b, r.stream});
-    S->to_free.push_back({tk, nullptr, nullptr});
+        if (b) to_free.push_back({0, b});
+    to_free.push_back({tk, nullptr});
     r.edges = nullptr;
     r.rowptr = nullptr;
     r.col = nullptr;
 }
 
-// Mark tickets done with `status` (lock held).  Failed requests give all their
-// memory back at once; finished ones give back their scratch share.
+// Mark the tickets of a group, launched or not, done with `status` (lock held).  Failed
+// requests give all their memory back at once; finished ones give back their scratch
+// share.
 void complete(pa_server *S, const std::vector<uint64_t> &tickets, int status, uint32_t batch_size,
               const uint32_t *csr_status = nullptr)
 {
@@ -222,43 +246,50 @@ void complete(pa_server *S, const std::vector<uint64_t> &tickets, int status, ui
         }
         S->done_order.emplace_back(t, tk);
     }
+    --S->active;
+    ++S->gave;
+    wake(S);
     S->cv_done.notify_all();
 }
 
-// A pool allocation, stream-ordered on s.  When the pool's free blocks are too
+// An allocation of a lane, ordered on its stream, before any of a group's work is
+// queued.  From its range; where that has no piece large enough and work in flight
+// will give some back, it fails if the caller can wait.  Otherwise from the range's
+// free pages moved together, else from the pool.  When the pool's free blocks are too
 // fragmented, its memory that is free and no longer in use goes back to the
 // device and the allocation is tried once more; the caller retries later
-// (after a completion) if that fails too.  Nothing here waits for the GPU.
-cudaError_t pool_alloc(cudaMemPool_t pool, void **p, uint64_t bytes, cudaStream_t s)
+// (after a completion) if that fails too.
+cudaError_t lane_alloc(LaneState &LS, void **p, uint64_t bytes, bool may_wait)
 {
-    cudaError_t e = cudaMallocFromPoolAsync(p, std::max<uint64_t>(bytes, 16), pool, s);
+    bytes = std::max<uint64_t>(bytes, 16);
+    *p = LS.range.take(bytes);
+    if (*p) return cudaSuccess;
+    const bool idle = LS.inflight.empty() && LS.retired.empty();
+    if (may_wait && !idle) return cudaErrorMemoryAllocation;
+    if (idle && cudaStreamSynchronize(LS.stream) == cudaSuccess) *p = LS.range.regroup(bytes);
+    if (*p) return cudaSuccess;
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, LS.pool, LS.stream);
     if (e != cudaSuccess) {
         (void)cudaGetLastError();
-        cudaMemPoolTrimTo(pool, 0);
-        e = cudaMallocFromPoolAsync(p, std::max<uint64_t>(bytes, 16), pool, s);
-        if (e != cudaSuccess) (void)cudaGetLastError();
+        cudaMemPoolTrimTo(LS.pool, 0);
+        e = cudaMallocFromPoolAsync(p, bytes, LS.pool, LS.stream);
+        if (e != cudaSuccess) {
+            (void)cudaGetLastError();
+            *p = nullptr;
+        }
     }
     return e;
 }
 
-// The lane's stream with the fewest launches in flight.
-cudaStream_t pick_stream(const LaneState &L)
+// Its end, in the stream's order: memory given back to the range is next used by work
+// queued later on the same stream.
+cudaError_t lane_free(LaneState &LS, void *p)
 {
-    cudaStream_t best = L.streams[0];
-    size_t best_n = SIZE_MAX;
-    for (cudaStream_t s : L.streams) {
-        size_t c = 0;
-        for (const Launch &x : L.inflight) c += x.stream == s;
-        if (c < best_n) {
-            best_n = c;
-            best = s;
-        }
-    }
-    return best;
+    return LS.range.give(p) ? cudaSuccess : cudaFreeAsync(p, LS.stream);
 }
 
 // Launch one group of admitted requests (same id width, all batchable) as a
-// batch, or one request alone, on the lane's least busy stream; then, with CSR
+// batch, or one request alone, on the lane's stream; then, with CSR
 // outputs, every request's CSR.  Called without the lock.  When an allocation
 // fails before anything is queued and may_defer is set, the partial
 // allocations are freed and false is returned: the caller keeps the group
@@ -267,15 +298,20 @@ bool launch_group(pa_server *S, const std::vector<Job> &jobs, bool batch, uint32
                   bool may_defer)
 {
     LaneState &LS = S->lanes[lane];
-    const cudaStream_t st = pick_stream(LS);
+    const cudaStream_t st = LS.stream;
+    {
+        std::lock_guard<std::mutex> lk(S->mu);
+        ++S->active;
+    }
     const uint32_t k = (uint32_t)jobs.size();
     const bool csr = (S->cfg.outputs & PA_OUT_CSR) != 0;
     const bool keep_pairs = (S->cfg.outputs & PA_OUT_PAIRS) != 0;
-    std::vector<void *> edges(k, nullptr), rowptr(k, nullptr), col(k, nullptr), cscr(k, nullptr);
+    std::vector<void *> edges(k, nullptr), rowptr(k, nullptr), col(k, nullptr);
+    void *cscr = nullptr;   // the CSR scratch of every request in turn, as large as the largest
+    uint64_t cscr_bytes = 0;
     std::vector<pa_params> prms(k);
     std::vector<uint64_t> ebytes(k);
     Launch L;
-    L.stream = st;
     for (uint32_t i = 0; i < k; ++i) {
         L.tickets.push_back(jobs[i].ticket);
         prms[i] = jobs[i].prm;
@@ -284,10 +320,12 @@ bool launch_group(pa_server *S, const std::vector<Job> &jobs, bool batch, uint32
     int rc = PA_OK;
     cudaError_t e = cudaSuccess;
     for (uint32_t i = 0; i < k && e == cudaSuccess; ++i) {
-        e = pool_alloc(LS.pool, &edges[i], ebytes[i], st);
-        if (csr && e == cudaSuccess) e = pool_alloc(LS.pool, &rowptr[i], jobs[i].rowptr_bytes, st);
-        if (csr && e == cudaSuccess) e = pool_alloc(LS.pool, &col[i], jobs[i].col_bytes, st);
+        e = lane_alloc(LS, &edges[i], ebytes[i], may_defer);
+        if (csr && e == cudaSuccess) e = lane_alloc(LS, &rowptr[i], jobs[i].rowptr_bytes, may_defer);
+        if (csr && e == cudaSuccess) e = lane_alloc(LS, &col[i], jobs[i].col_bytes, may_defer);
+        cscr_bytes = std::max(cscr_bytes, jobs[i].csr_scratch);
     }
+    if (csr && e == cudaSuccess) e = lane_alloc(LS, &cscr, cscr_bytes, may_defer);
     BatchJob J;
     uint64_t scratch_bytes = 0, image_bytes = 0;
     if (e == cudaSuccess) {
@@ -298,20 +336,23 @@ bool launch_group(pa_server *S, const std::vector<Job> &jobs, bool batch, uint32
         } else {
             rc = pa_scratch_bytes(&prms[0], &scratch_bytes);
         }
-        if (rc == PA_OK) e = pool_alloc(LS.pool, &L.scratch, scratch_bytes, st);
+        if (rc == PA_OK) e = lane_alloc(LS, &L.scratch, scratch_bytes, may_defer);
     }
     if (e != cudaSuccess && may_defer) {
         // nothing queued yet: give the memory back (stream-ordered) and wait
         for (uint32_t i = 0; i < k; ++i)
             for (void *b : {edges[i], rowptr[i], col[i]})
-                if (b) cudaFreeAsync(b, st);
-        if (L.scratch) cudaFreeAsync(L.scratch, st);
+                if (b) lane_free(LS, b);
+        if (cscr) lane_free(LS, cscr);
+        if (L.scratch) lane_free(LS, L.scratch);
+        std::lock_guard<std::mutex> lk(S->mu);
+        --S->active;
         return false;
     }
     if (e != cudaSuccess && rc == PA_OK) rc = set_cuda_error(e);
     if (rc == PA_OK) {
         L.status_off = (image_bytes + 15) & ~15ull;
-        L.buf = get_pinned(S, L.status_off + 4ull * (k + 1));
+        L.buf = get_pinned(LS, L.status_off + 4ull * (k + 1));
         if (!L.buf.p) rc = PA_ERR_OOM;
     }
     bool queued = false;   // work that reads the pinned image or the scratch is queued
@@ -329,8 +370,8 @@ bool launch_group(pa_server *S, const std::vector<Job> &jobs, bool batch, uint32
                             sizeof(uint32_t), cudaMemcpyDeviceToHost, st);
         if (e != cudaSuccess) rc = set_cuda_error(e);
     }
-    // CSR of every request, in the same stream; its scratch (and the pairs when
-    // they are not kept) is freed in stream order behind it
+    // CSR of every request, in the same stream; the pairs when they are not kept, and
+    // the scratch at the end, are freed in stream order behind it
     uint32_t *csr_status = L.buf.p ? reinterpret_cast<uint32_t *>(L.buf.p + L.status_off) + 1
                                    : nullptr;
     for (uint32_t i = 0; i < k && rc == PA_OK; ++i) {
@@ -338,23 +379,21 @@ bool launch_group(pa_server *S, const std::vector<Job> &jobs, bool batch, uint32
             csr_status[i] = PA_OK;
             continue;
         }
-        e = pool_alloc(LS.pool, &cscr[i], jobs[i].csr_scratch, st);
-        if (e != cudaSuccess) {
-            rc = set_cuda_error(e);
-            break;
-        }
         uint64_t err_off = 0;
-        rc = csr_enqueue(&prms[i], edges[i], (int64_t *)rowptr[i], col[i], cscr[i],
-                         jobs[i].csr_scratch, st, &err_off);
+        rc = csr_enqueue(&prms[i], edges[i], (int64_t *)rowptr[i], col[i], cscr, cscr_bytes, st,
+                         &err_off);
         if (rc != PA_OK) break;
-        e = cudaMemcpyAsync(csr_status + i, (const unsigned char *)cscr[i] + err_off, 4,
+        e = cudaMemcpyAsync(csr_status + i, (const unsigned char *)cscr + err_off, 4,
                             cudaMemcpyDeviceToHost, st);
-        if (e == cudaSuccess) e = cudaFreeAsync(cscr[i], st);
-        cscr[i] = nullptr;
         if (e == cudaSuccess && !keep_pairs) {
-            e = cudaFreeAsync(edges[i], st);
+            e = lane_free(LS, edges[i]);
             edges[i] = nullptr;
         }
+        if (e != cudaSuccess) rc = set_cuda_error(e);
+    }
+    if (rc == PA_OK && cscr) {
+        e = lane_free(LS, cscr);
+        cscr = nullptr;
         if (e != cudaSuccess) rc = set_cuda_error(e);
     }
     if (rc == PA_OK) {
@@ -370,15 +409,15 @@ bool launch_group(pa_server *S, const std::vector<Job> &jobs, bool batch, uint32
             L.done = nullptr;
         }
         Retired R;
-        R.stream = st;
         R.buf = L.buf;
         if (L.scratch) R.device.push_back(L.scratch);
-        for (void *b : cscr)
-            if (b) R.device.push_back(b);
+        if (cscr) R.device.push_back(cscr);
         bool parked = false;
         if (queued && cudaEventCreateWithFlags(&R.done, cudaEventDisableTiming) == cudaSuccess) {
             if (cudaEventRecord(R.done, st) == cudaSuccess) {
-                S->retired.push_back(R);
+                LS.retired.push_back(R);
+                std::lock_guard<std::mutex> lk(S->mu);
+                ++S->active;
                 parked = true;
             } else {
                 cudaEventDestroy(R.done);
@@ -387,11 +426,8 @@ bool launch_group(pa_server *S, const std::vector<Job> &jobs, bool batch, uint32
         if (!parked) {
             // nothing queued (or no event to wait on): the stream orders the frees
             if (queued) cudaStreamSynchronize(st);   // last resort: no event could be made
-            for (void *b : R.device) cudaFreeAsync(b, st);
-            if (R.buf.p) {
-                std::lock_guard<std::mutex> lk(S->mu);
-                S->pinned_free.push_back(R.buf);
-            }
+            for (void *b : R.device) lane_free(LS, b);
+            if (R.buf.p) LS.pinned_free.push_back(R.buf);
         }
         L.buf = Pinned{};
     }
@@ -402,7 +438,6 @@ bool launch_group(pa_server *S, const std::vector<Job> &jobs, bool batch, uint32
         it->second.edges = edges[i];
         it->second.rowptr = (int64_t *)rowptr[i];
         it->second.col = col[i];
-        it->second.stream = st;
     }
     ++S->st.batches;
     if (rc == PA_OK) {
@@ -434,68 +469,62 @@ std::vector<std::pair<std::vector<Job>, bool>> make_groups(pa_server *S, const u
     return out;
 }
 
-bool anything_in_flight(const pa_server *S)
-{
-    for (const LaneState &L : S->lanes)
-        if (!L.inflight.empty()) return true;
-    return !S->retired.empty();
-}
-
-void control_loop(pa_server *S)
+void control_loop(pa_server *S, uint32_t lane)
 {
     cudaSetDevice(S->device);
+    LaneState &LS = S->lanes[lane];
     const uint32_t max_batch = S->cfg.max_batch ? S->cfg.max_batch : 4096u;
     const uint32_t max_inflight = S->cfg.max_inflight ? S->cfg.max_inflight : 4u;
     std::vector<uint64_t> adm(max_batch);
     for (;;) {
-        bool progressed = false, freed = false;
-        // 1. completions (each stream runs its launches in order; streams in any order)
-        for (LaneState &LS : S->lanes) {
-            for (size_t i = 0; i < LS.inflight.size();) {
-                Launch &L = LS.inflight[i];
-                const cudaError_t q = cudaEventQuery(L.done);
-                if (q == cudaErrorNotReady) {
-                    ++i;
-                    continue;
-                }
-                int status = PA_OK;
-                if (q != cudaSuccess) {
-                    status = set_cuda_error(q);
-                } else {
-                    uint32_t dev_status = 0;
-                    std::memcpy(&dev_status, L.buf.p + L.status_off, sizeof(dev_status));
-                    status = (int)dev_status;
-                }
-                cudaFreeAsync(L.scratch, L.stream);
-                cudaEventDestroy(L.done);
-                {
-                    std::lock_guard<std::mutex> lk(S->mu);
-                    S->pinned_free.push_back(L.buf);
-                    complete(S, L.tickets, status, (uint32_t)L.tickets.size(),
-                             reinterpret_cast<const uint32_t *>(L.buf.p + L.status_off) + 1);
-                }
-                LS.inflight.erase(LS.inflight.begin() + (ptrdiff_t)i);
-                progressed = freed = true;
+        bool progressed = false;
+        // 1. completions (the stream runs its launches in order)
+        for (size_t i = 0; i < LS.inflight.size();) {
+            Launch &L = LS.inflight[i];
+            const cudaError_t q = cudaEventQuery(L.done);
+            if (q == cudaErrorNotReady) {
+                ++i;
+                continue;
             }
+            int status = PA_OK;
+            if (q != cudaSuccess) {
+                status = set_cuda_error(q);
+            } else {
+                uint32_t dev_status = 0;
+                std::memcpy(&dev_status, L.buf.p + L.status_off, sizeof(dev_status));
+                status = (int)dev_status;
+            }
+            lane_free(LS, L.scratch);
+            cudaEventDestroy(L.done);
+            {
+                std::lock_guard<std::mutex> lk(S->mu);
+                complete(S, L.tickets, status, (uint32_t)L.tickets.size(),
+                         reinterpret_cast<const uint32_t *>(L.buf.p + L.status_off) + 1);
+            }
+            LS.pinned_free.push_back(L.buf);
+            LS.inflight.erase(LS.inflight.begin() + (ptrdiff_t)i);
+            progressed = true;
         }
-        for (size_t i = 0; i < S->retired.size();) {
-            Retired &R = S->retired[i];
+        for (size_t i = 0; i < LS.retired.size();) {
+            Retired &R = LS.retired[i];
             if (cudaEventQuery(R.done) == cudaErrorNotReady) {
                 ++i;
                 continue;
             }
-            for (void *b : R.device) cudaFreeAsync(b, R.stream);
+            for (void *b : R.device) lane_free(LS, b);
             cudaEventDestroy(R.done);
-            if (R.buf.p) {
-                std::lock_guard<std::mutex> lk(S->mu);
-                S->pinned_free.push_back(R.buf);
-            }
-            S->retired.erase(S->retired.begin() + (ptrdiff_t)i);
-            progressed = freed = true;
+            if (R.buf.p) LS.pinned_free.push_back(R.buf);
+            LS.retired.erase(LS.retired.begin() + (ptrdiff_t)i);
+            std::lock_guard<std::mutex> lk(S->mu);
+            --S->active;
+            ++S->gave;
+            wake(S);
+            progressed = true;
         }
         // 2. released and expired buffers
-        std::vector<pa_server::Free> frees;
+        std::vector<Free> frees;
         bool stopping;
+        uint64_t seen;
         {
             std::lock_guard<std::mutex> lk(S->mu);
             if (S->cfg.ttl_ns) {
@@ -506,53 +535,64 @@ void control_loop(pa_server *S)
                     auto it = S->reqs.find(tk);
                     if (it == S->reqs.end() || it->second.state != RQ_DONE) continue;
                     drop_buffers(S, tk, it->second);
+                    if (it->second.lane != lane) wake(S);
                     S->reqs.erase(it);
                     ++S->st.expired;
                 }
             } else {
                 S->done_order.clear();
             }
-            frees.swap(S->to_free);
+            frees.swap(LS.to_free);
             stopping = S->stop;
+            seen = S->events;
         }
         for (auto &f : frees) {
-            if (f.ptr) cudaFreeAsync(f.ptr, f.stream ? f.stream : S->lanes[kBulk].streams[0]);
+            if (f.ptr) lane_free(LS, f.ptr);
             if (f.ticket) pa_sched_release(S->sched, f.ticket, UINT64_MAX);
-            progressed = freed = true;
+            progressed = true;
+        }
+        if (!frees.empty()) {
+            std::lock_guard<std::mutex> lk(S->mu);
+            ++S->gave;
+            wake(S);
         }
         // 3. groups whose allocations failed: retried once memory has come back,
         // failed when nothing is left in flight to give any back
-        for (uint32_t lane = 0; lane < kLanes; ++lane) {
-            LaneState &LS = S->lanes[lane];
-            while (!LS.deferred.empty() && LS.inflight.size() < max_inflight) {
-                auto &g = LS.deferred.front();
+        while (!LS.deferred.empty() && LS.inflight.size() < max_inflight) {
+            auto &g = LS.deferred.front();
+            bool busy;
+            uint64_t gave;
+            {
+                std::lock_guard<std::mutex> lk(S->mu);
                 if (stopping) {
                     std::vector<uint64_t> tks;
                     for (const Job &jb : g.first) tks.push_back(jb.ticket);
-                    std::lock_guard<std::mutex> lk(S->mu);
+                    ++S->active;   // complete() takes a group out
                     complete(S, tks, PA_ERR_OOM, (uint32_t)tks.size());
-                } else {
-                    const bool busy = anything_in_flight(S);
-                    if (busy && !freed) break;
-                    if (!launch_group(S, g.first, g.second, lane, busy)) break;
                 }
-                LS.deferred.pop_front();
-                progressed = true;
+                busy = S->active > 0;
+                gave = S->gave;
             }
+            if (!stopping) {
+                if (busy && gave == LS.deferred_at) break;
+                if (!launch_group(S, g.first, g.second, lane, busy)) {
+                    LS.deferred_at = gave;
+                    break;
+                }
+            }
+            LS.deferred.pop_front();
+            progressed = true;
         }
-        if (stopping && !anything_in_flight(S) && S->lanes[kBulk].deferred.empty() &&
-            S->lanes[kExpress].deferred.empty())
-            break;
-        // 4. admission, lane by lane
-        for (uint32_t lane = 0; lane < kLanes && !stopping; ++lane) {
-            LaneState &LS = S->lanes[lane];
-            if (LS.inflight.size() >= max_inflight || !LS.deferred.empty()) continue;
+        if (stopping && LS.inflight.empty() && LS.retired.empty() && LS.deferred.empty()) break;
+        // 4. admission
+        if (!stopping && LS.inflight.size() < max_inflight && LS.deferred.empty()) {
             std::vector<std::pair<std::vector<Job>, bool>> groups;
             {
                 std::lock_guard<std::mutex> lk(S->mu);
                 const uint64_t t = S->now();
                 const uint32_t n = pa_sched_admit_lanes(S->sched, t, adm.data(), max_batch, 1u << lane);
                 groups = make_groups(S, adm.data(), n, t);
+                LS.deferred_at = S->gave;
             }
             for (auto &g : groups) {
                 if (!LS.deferred.empty() || !launch_group(S, g.first, g.second, lane, true))
@@ -563,27 +603,25 @@ void control_loop(pa_server *S)
         // 5. sleep
         if (!progressed) {
             std::unique_lock<std::mutex> lk(S->mu);
-            if (!anything_in_flight(S))
-                S->cv_work.wait_for(lk, std::chrono::milliseconds(2));
-            else
-                S->cv_work.wait_for(lk, std::chrono::microseconds(20));
+            const bool idle = LS.inflight.empty() && LS.retired.empty();
+            S->cv_work.wait_for(lk, std::chrono::microseconds(idle ? 2000 : 20),
+                                [&] { return S->events != seen; });
         }
     }
-    // shutdown: every launch has completed; free what is still held
+    // shutdown: every launch of the lane has completed; free what it still holds
     {
         std::lock_guard<std::mutex> lk(S->mu);
-        for (auto &kv : S->reqs)
-            for (void *b : {kv.second.edges, (void *)kv.second.rowptr, kv.second.col})
-                if (b) cudaFreeAsync(b, kv.second.stream ? kv.second.stream
-                                                         : S->lanes[kBulk].streams[0]);
-        S->reqs.clear();
-        for (auto &f : S->to_free)
-            if (f.ptr) cudaFreeAsync(f.ptr, f.stream ? f.stream : S->lanes[kBulk].streams[0]);
-        S->to_free.clear();
+        for (auto &kv : S->reqs) {
+            if (kv.second.lane != lane) continue;
+            drop_buffers(S, kv.first, kv.second);
+        }
+        for (auto &f : LS.to_free)
+            if (f.ptr) lane_free(LS, f.ptr);
+        LS.to_free.clear();
+        if (--S->running == 0) S->reqs.clear();
         S->cv_done.notify_all();
     }
-    for (const LaneState &LS : S->lanes)
-        for (cudaStream_t s : LS.streams) cudaStreamSynchronize(s);
+    cudaStreamSynchronize(LS.stream);
 }
 
 }  // namespace
@@ -620,7 +658,7 @@ int pa_server_create(const pa_server_config *cfg, pa_server **out)
         cudaStream_t s = nullptr;
         e = cudaStreamCreateWithPriority(&s, cudaStreamNonBlocking,
                                          lane == kExpress ? greatest : least);
-        if (e == cudaSuccess) LS.streams.push_back(s);
+        if (e == cudaSuccess) LS.stream = s;
         if (e == cudaSuccess) {
             cudaMemPoolProps props;
             std::memset(&props, 0, sizeof(props));
@@ -636,7 +674,8 @@ int pa_server_create(const pa_server_config *cfg, pa_server **out)
     }
     auto destroy_lanes = [&] {
         for (LaneState &LS : S->lanes) {
-            for (cudaStream_t s : LS.streams) cudaStreamDestroy(s);
+            for (auto &b : LS.pinned_free) cudaFreeHost(b.p);
+            if (LS.stream) cudaStreamDestroy(LS.stream);
             if (LS.pool) cudaMemPoolDestroy(LS.pool);
         }
     };
@@ -655,28 +694,46 @@ int pa_server_create(const pa_server_config *cfg, pa_server **out)
         delete S;
         return PA_ERR_OOM;
     }
-    // Map each lane's share of the budget into its pool now (allocated once and
-    // freed; the pool keeps freed memory), so that serving does not grow the
-    // pools -- a driver mapping on the control thread -- while requests wait.
-    // The express lane's requests are small: an eighth of the budget.
+    // Each lane's share of the budget, mapped now.  The express lane's requests are
+    // small: an eighth of the budget.
     if (S->cfg.budget_bytes) {
         cudaSetDevice(S->device);
         for (uint32_t lane = 0; lane < kLanes; ++lane) {
-            LaneState &LS = S->lanes[lane];
             const uint64_t share = lane == kExpress ? S->cfg.budget_bytes / 8
                                                     : S->cfg.budget_bytes - S->cfg.budget_bytes / 8;
-            void *p = nullptr;
-            if (cudaMallocFromPoolAsync(&p, share, LS.pool, LS.streams[0]) == cudaSuccess)
-                cudaFreeAsync(p, LS.streams[0]);
-            else
-                (void)cudaGetLastError();   // best effort: the pool grows on demand instead
-            cudaStreamSynchronize(LS.streams[0]);
+            S->lanes[lane].range.open(S->device, share);   // or the pool does it all, on demand
+        }
+        // staging for the express lane's launches: pinning memory is a driver mapping too
+        const uint32_t launches = S->cfg.max_inflight ? S->cfg.max_inflight : 4u;
+        for (uint32_t i = 0; i < std::min(launches, 16u); ++i) {
+            Pinned b;
+            b.cap = kPinnedBytes;
+            if (cudaMallocHost(&b.p, b.cap) != cudaSuccess) {
+                (void)cudaGetLastError();   // made on demand instead
+                break;
+            }
+            S->lanes[kExpress].pinned_free.push_back(b);
         }
         cudaSetDevice(prev);
     }
     S->st.budget_bytes = S->cfg.budget_bytes;
     S->t0 = std::chrono::steady_clock::now();
-    S->worker = std::thread(control_loop, S);
+    for (uint32_t lane = 0; lane < kLanes; ++lane) {
+        {
+            std::lock_guard<std::mutex> lk(S->mu);
+            ++S->running;
+        }
+        try {
+            S->lanes[lane].worker = std::thread(control_loop, S, lane);
+        } catch (const std::system_error &) {
+            {
+                std::lock_guard<std::mutex> lk(S->mu);
+                --S->running;
+            }
+            pa_server_destroy(S);
+            return PA_ERR_OOM;
+        }
+    }
     *out = S;
     return PA_OK;
 }
@@ -712,7 +769,7 @@ int pa_server_submit(pa_server *S, const pa_params *prm, uint64_t *ticket)
     S->reqs.emplace(tk, r);
     ++S->st.submitted;
     *ticket = tk;
-    S->cv_work.notify_one();
+    wake(S);
     return PA_OK;
 }
 
@@ -778,7 +835,7 @@ int pa_server_release(pa_server *S, uint64_t ticket)
         drop_buffers(S, ticket, r);
     S->reqs.erase(it);
     ++S->st.released;
-    S->cv_work.notify_one();
+    wake(S);
     return PA_OK;
 }
 
@@ -802,12 +859,14 @@ int pa_server_destroy(pa_server *S)
     {
         std::lock_guard<std::mutex> lk(S->mu);
         S->stop = true;
-        S->cv_work.notify_all();
+        wake(S);
     }
-    if (S->worker.joinable()) S->worker.join();
-    for (auto &b : S->pinned_free) cudaFreeHost(b.p);
+    for (LaneState &LS : S->lanes)
+        if (LS.worker.joinable()) LS.worker.join();
     for (LaneState &LS : S->lanes) {
-        for (cudaStream_t s : LS.streams) cudaStreamDestroy(s);
+        for (auto &b : LS.pinned_free) cudaFreeHost(b.p);
+        LS.range.close();
+        cudaStreamDestroy(LS.stream);
         cudaMemPoolDestroy(LS.pool);
     }
     pa_sched_destroy(S->sched);

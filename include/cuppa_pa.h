@@ -260,18 +260,19 @@ int pa_batch_generate(const pa_params *prms, uint32_t count, void *const *d_edge
 
 /* ---- request server ------------------------------------------------------------ */
 /* A served stream of independent generation requests (no counterpart in the
- * reference, which makes one graph per process run, src/main.cu:105-116).  One
- * control thread per server owns its CUDA streams on its device: it admits
+ * reference, which makes one graph per process run, src/main.cu:105-116).  Two
+ * lanes, each with a control thread and a CUDA stream: the thread admits
  * queued requests while their device memory (edge buffer + generation scratch)
  * fits the budget, launches everything admitted as one batch
- * (pa_batch_generate's launches) whenever a lane has fewer than max_inflight
+ * (pa_batch_generate's launches) whenever the lane has fewer than max_inflight
  * batches on the GPU -- so requests that arrive while a batch runs form the
  * next one -- and marks each request done when its batch's completion event
- * has fired; it never waits on the GPU.  Two lanes share the budget: requests
+ * has fired; it never waits on the GPU.  The lanes share the budget: requests
  * of at most express_edges edges run in the express lane, on a stream of the
- * device's highest priority with a memory pool of its own, so a small request
- * that arrives while a large batch runs starts at that batch's next kernel
- * boundary; a lane's launches queue in order on its stream.
+ * device's highest priority, so a small request that arrives while a large batch
+ * runs starts as that batch's blocks end; a lane's launches queue in order on its
+ * stream.  Each lane hands out a share of the budget mapped when the server starts (an
+ * eighth for the express lane) and asks the driver for more only where that does not do.
  * A result stays in device memory, owned by the server, until
  * pa_server_release (or until it has been finished for ttl_ns).  Submit, poll,
  * wait and release may be called from any thread. */
@@ -322,7 +323,7 @@ typedef struct pa_server_stats {
 } pa_server_stats;
 
 int pa_server_config_init(pa_server_config *cfg);
-/* Start a server (its control thread and stream); *out gets the handle. */
+/* Start a server (its lanes' threads, streams and memory); *out gets the handle. */
 int pa_server_create(const pa_server_config *cfg, pa_server **out);
 /* Queue a request (a copy of *prm is kept; id widths may differ between
  * requests).  PA_ERR_CAPACITY: it can never fit the budget; PA_ERR_BUSY: the
@@ -339,7 +340,7 @@ int pa_server_wait(pa_server *srv, uint64_t ticket, uint64_t timeout_ns, pa_resu
  * completed. */
 int pa_server_release(pa_server *srv, uint64_t ticket);
 int pa_server_stats_get(pa_server *srv, pa_server_stats *out);
-/* Stop the control thread, wait for the GPU work, free everything.  No other
+/* Stop the control threads, wait for the GPU work, free everything.  No other
  * thread may be inside a pa_server_* call on this handle. */
 int pa_server_destroy(pa_server *srv);
 
