@@ -1,6 +1,8 @@
 // pa_post.cu -- passes over a generated edge list: row canonicalisation and
 // undirected degrees (the device side of src/PA/cuPPA/cuPPA.cu:103-165, which
 // copies the whole graph to the host and counts there).
+#include <algorithm>
+
 #include "pa_device.cuh"
 #include "pa_internal.h"
 #include "pa_wide.h"
@@ -69,6 +71,11 @@ __global__ void canon_kernel(const Id *in, Id *out, uint64_t n, uint32_t d, uint
 // (64-bit counts for lists of 2^31 pairs and more, and below kDegNarrow nodes,
 // whose 64-bit counts are in L2 too and need no widening launches).  Early nodes hold the
 // hubs: ids below kLowIds are counted in shared memory, one flush per block.
+//
+// Seed edges: SLOTS lists hold none, and the counts start with them; those of PAIRS
+// lists are spread over the grid like the rest.  A clique's source repeats through its
+// row, so a warp counts equal sources with one atomic (d = 8,192, n = 2 d, 3.4 * 10^7
+// seed edges: 36.4 ms by one block, 0.45 so).
 // n = 2^24, d = 8, p = 0.3, 32-bit ids: 5.63 -> 0.97 ms (138 G targets/s; two
 // atomics a pair combined by __match_any_sync before); p = 0.1, 64-bit ids:
 // 15.9 -> 0.82 ms; n = 10^6: 0.309 -> 0.062 ms.
@@ -78,42 +85,56 @@ constexpr uint32_t kDegChunk = 8192;   // pairs per block step at most
 constexpr uint64_t kDegNarrow = 1ull << 22;   // nodes above which 32-bit counts pay
 constexpr uint32_t kLowIds = 8192;     // 32 KB of shared counters
 
+// The counts before any pair is read: d out-edges of a generated node, and with `seeds`
+// the seed edges, both ends (CLIQUE: every seed node has d; STAR_REF: node d has d, the
+// others 1).
 template <typename Cnt>
 __global__ void __launch_bounds__(kDegThreads) degree_init_kernel(Cnt *deg, uint64_t n, uint64_t u_first,
-                                                                  uint32_t d)
+                                                                  uint32_t d, bool seeds,
+                                                                  uint32_t seed_mode)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    const Cnt low = !seeds ? 0 : (seed_mode == PA_SEED_CLIQUE ? (Cnt)d : (Cnt)1);
     for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += stride)
-        deg[u] = u >= u_first ? (Cnt)d : (Cnt)0;
+        deg[u] = u >= u_first || (seeds && u == d) ? (Cnt)d : low;
 }
 
 // Pairs (or, with Slots, targets) of the generated nodes: `count` of them from E
-// + (Slots ? 0 : 2) * seed_edges, `chunk` (<= kDegChunk) a block step; block 0 also
-// counts the seed edges.
+// + (Slots ? 0 : 2) * seed_edges, `chunk` (<= kDegChunk) a block step; with pairs the
+// seed edges too.
 template <typename Id, bool Slots, typename Cnt>
 __global__ void __launch_bounds__(kDegThreads) degree_kernel(const Id *E, uint64_t count,
                                                              uint32_t chunk, uint32_t d,
                                                              uint32_t d_inv, uint64_t u_first,
-                                                             uint32_t seed_mode, uint64_t seed_edges,
+                                                             uint64_t seed_edges,
                                                              uint64_t n, bool vec, Cnt *deg)
 {
     __shared__ uint32_t low[kLowIds];
     for (uint32_t i = threadIdx.x; i < kLowIds; i += kDegThreads) low[i] = 0;
     __syncthreads();
-    if (blockIdx.x == 0)
-        for (uint64_t e = threadIdx.x; e < seed_edges; e += kDegThreads) {
-            uint64_t s, t;
-            if constexpr (Slots) {
-                seed_edge_of(e, d, seed_mode, s, t);
-            } else {
-                s = (uint64_t)E[2 * e];
-                t = (uint64_t)E[2 * e + 1];
+    if constexpr (!Slots) {
+        const uint64_t step = (uint64_t)gridDim.x * kDegThreads;
+        const uint32_t lane = threadIdx.x & 31u;
+        for (uint64_t e0 = (uint64_t)blockIdx.x * kDegThreads + (threadIdx.x - lane); e0 < seed_edges;
+             e0 += step) {
+            const uint64_t e = e0 + lane;
+            uint64_t s = ~0ull, t = ~0ull;
+            if (e < seed_edges) {
+                s = (uint64_t)(int64_t)E[2 * e];
+                t = (uint64_t)(int64_t)E[2 * e + 1];
             }
-            if (s < n && t < n) {   // ids are used as addresses: never trust them
-                atomicAdd(deg + s, (Cnt)1);
-                atomicAdd(deg + t, (Cnt)1);
+            const bool in = s < n && t < n;   // ids are used as addresses: never trust them
+            const uint32_t same = __match_any_sync(kFull, in ? s : ~0ull);
+            if (in && (uint32_t)__ffs(same) - 1u == lane) {
+                if (s < kLowIds) atomicAdd(low + s, (uint32_t)__popc(same));
+                else atomicAdd(deg + s, (Cnt)__popc(same));
+            }
+            if (in) {
+                if (t < kLowIds) atomicAdd(low + t, 1u);
+                else atomicAdd(deg + t, (Cnt)1);
             }
         }
+    }
     const Id *G = E + (Slots ? 0 : 2 * seed_edges);
     constexpr uint32_t U = 4;   // loads in flight per thread
     for (uint64_t c0 = (uint64_t)blockIdx.x * chunk; c0 < count; c0 += (uint64_t)gridDim.x * chunk) {
@@ -273,7 +294,8 @@ template <typename Id, bool Slots, typename Cnt>
 void degrees_launch(const pa_params *prm, const GenPlan &p, const Id *E, Cnt *deg, cudaStream_t s)
 {
     const uint64_t n = prm->n, count = (n - p.u_first) * prm->d;
-    degree_init_kernel<Cnt><<<grid_for(n, kDegThreads), kDegThreads, 0, s>>>(deg, n, p.u_first, prm->d);
+    degree_init_kernel<Cnt><<<grid_for(n, kDegThreads), kDegThreads, 0, s>>>(deg, n, p.u_first, prm->d,
+                                                                             Slots, prm->seed_mode);
     // floor(x / d) = umulhi(x, d_inv) for x below 2^16: d_inv = ceil(2^32 / d) is off
     // by less than 1 / x (d = 1: 2^32 does not fit)
     // one load per pair when the pairs are aligned to their size
@@ -282,8 +304,10 @@ void degrees_launch(const pa_params *prm, const GenPlan &p, const Id *E, Cnt *de
     // whole chunks, four blocks per SM; less per block step where that leaves SMs idle
     uint32_t chunk = kDegChunk;
     while (chunk > 1024 && count < 600ull * chunk) chunk /= 2;
-    degree_kernel<Id, Slots, Cnt><<<grid_for(count, chunk, 4), kDegThreads, 0, s>>>(
-        E, count, chunk, prm->d, d_inv, p.u_first, prm->seed_mode, p.seed_edges, n, vec, deg);
+    const uint64_t blocks = std::max<uint64_t>((count + chunk - 1) / chunk,
+                                               Slots ? 0 : p.seed_edges / (4 * kDegThreads));
+    degree_kernel<Id, Slots, Cnt><<<grid_for(blocks, 1, 4), kDegThreads, 0, s>>>(
+        E, count, chunk, prm->d, d_inv, p.u_first, p.seed_edges, n, vec, deg);
 }
 
 template <typename Id>
