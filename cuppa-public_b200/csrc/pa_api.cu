@@ -18,6 +18,8 @@ static thread_local int g_last_cuda_error = 0;
 
 int set_cuda_error(cudaError_t e)
 {
+    // reported here: the runtime's own record of it must not be read as the next call's
+    (void)cudaGetLastError();
     g_last_cuda_error = (int)e;
     if (e == cudaErrorMemoryAllocation) return PA_ERR_OOM;
     return PA_ERR_CUDA;
