@@ -46,7 +46,6 @@ from __future__ import annotations
 
 import argparse
 import json
-import math
 import os
 import statistics
 import subprocess
@@ -511,14 +510,6 @@ def run_gpu(args, w):
             kernel, k_edges, kern_s = "start_kernel", start_edges, statistics.mean(start_ms) / 1e3
         achieved = k_edges * bpe / kern_s / 1e9
         traffic = load_traffic(args.workload)     # ncu DRAM bytes of one such launch
-        # set-up kernel, start kernel (a launch per range of nodes, doubling from 2^21, in
-        # graphs that draw copied slots again), tile kernel
-        nodes = u_split - (w["d"] + 1)
-        p_eff = 0.5 if w.get("model", COPY) == BA else w["p"]
-        hops = (gen_edges <= 0 and 0.4 <= p_eff <= 0.6
-                and nodes * w["d"] * 2 * (w["id_bits"] // 8) >= 2_000_000_000)
-        launches = ((1 + (1 + math.ceil(math.log2(nodes / 2 ** 21)) if hops else 1)
-                     if nodes > 0 else 0) + (1 if gen_edges > 0 else 0))
         line = {
             "metric": w.get("metric", METRIC), "value": value, "unit": "edges/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps,
@@ -544,7 +535,7 @@ def run_gpu(args, w):
                                "start_split_node": u_split},
             "e2e": e2e,
             "e2e_cuda_graph": e2e_graph,
-            "gpu_launches": launches * args.steps,
+            "gpu_launches": pa.generate_launches(prm) * args.steps,
             "clocks": clk.summary(),
             "device_stats": st.as_dict(),
             "parity": parity,
@@ -675,8 +666,8 @@ def run_stream(args):
         "e2e": {"value": E / e2e_s, "unit": "edges/s", "h2d_bytes_per_step": 80,
                 "d2h_bytes_per_step": nbytes,
                 "call": "pa_generate_to_file(prm, '/dev/null', TEXT): alloc, generate, write, free"},
-        # per step: the start kernel, then 3 formatting kernels per chunk
-        "gpu_launches": (1 + 3 * stream_chunks(w["n"], w["d"])) * args.steps,
+        # per step: the generation's, then 3 formatting kernels per chunk
+        "gpu_launches": (pa.generate_launches(prm) + 3 * stream_chunks(w["n"], w["d"])) * args.steps,
         "clocks": clk.summary(),
     }
     if not args.no_cpu_baseline:
@@ -949,7 +940,9 @@ def measure_served(args, rate: float, seconds: float, outputs_name: str, world: 
         "express_sized": pcts(True), "bulk_sized": pcts(False),
         "all_ok": ok, "server_stats_rank0": st,
         "statuses_rank0": {str(c): statuses.count(c) for c in sorted(set(statuses))},
-        "gpu_launches": st["batches"] * 2 + (st["completed"] * 6 if outputs & pa.PA_OUT_CSR else 0),
+        # a batch's fill and start kernel, then each request's CSR (warm-up requests too)
+        "gpu_launches": st["batches"] * 2 + (sum(map(pa.csr_launches, prms + prms[: args.warmup]))
+                                             if outputs & pa.PA_OUT_CSR else 0),
         "clocks": clk.summary(),
     }
     return fig, ok

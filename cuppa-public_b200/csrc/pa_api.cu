@@ -181,6 +181,16 @@ int pa_start_split(const pa_params *prm, uint64_t *u_split)
     return PA_OK;
 }
 
+int pa_generate_launches(const pa_params *prm, uint32_t *kernels)
+{
+    GenPlan p;
+    const int rc = make_plan(prm, &p);
+    if (rc != PA_OK) return rc;
+    if (!kernels) return PA_ERR_INVALID;
+    *kernels = generate_launches(prm, p);
+    return PA_OK;
+}
+
 int pa_scratch_bytes(const pa_params *prm, uint64_t *bytes)
 {
     GenPlan p;

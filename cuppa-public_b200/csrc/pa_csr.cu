@@ -1092,6 +1092,21 @@ int pa_csr_bytes(const pa_params *prm, uint64_t *rowptr_bytes, uint64_t *col_byt
     return PA_OK;
 }
 
+int pa_csr_launches(const pa_params *prm, uint32_t *kernels)
+{
+    GenPlan p;
+    const int rc = make_plan(prm, &p);
+    if (rc != PA_OK) return rc;
+    if (!kernels) return PA_ERR_INVALID;
+    if (!csr_supported(prm->n) || p.slots || (p.wide && prm->d > gen::kWideRankMaxD))
+        return PA_ERR_NOT_SUPPORTED;
+    const CsrLayout L = csr_layout(prm->n, prm->d, p.n_edges, p.id_bytes);
+    // histogram and passes of the sort; then row starts, rows and the listed chunks' in
+    // parts, or (d > 32) in parts, seed rows' and generated rows' out parts
+    *kernels = (p.n_edges > 0 ? 1 + L.passes : 0) + 3;
+    return PA_OK;
+}
+
 int pa_build_csr(const pa_params *prm, const void *d_edges, int64_t *d_rowptr, void *d_col,
                  void *d_scratch, uint64_t scratch_bytes, void *stream)
 {

@@ -449,6 +449,57 @@ int fill_prefill(const pa_params *prm, const GenPlan &plan, void *d_edges, cudaS
     return e == cudaSuccess ? PA_OK : set_cuda_error(e);
 }
 
+namespace {
+
+// The start kernel's launches for one graph.
+struct StartRoute {
+    bool alone;                  // it generates every node
+    StartVariant variant;
+    uint64_t tile_nodes, tiles;  // of all launches
+    uint64_t first_tiles;        // of the first one; each later one doubles the tiles done
+    uint32_t launches;
+};
+
+// The filter and the launches' counters lie where tile flags would, unused in hop
+// launches.
+constexpr uint64_t kHopBytes = kHopFilterBytes + kHopMaxLaunches * kStartAreaBytes;
+
+// Tiles done after launch l (0, 1, ..).
+uint64_t tiles_after(const StartRoute &r, uint32_t l)
+{
+    return l + 1 < kHopMaxLaunches ? std::min(r.tiles, r.first_tiles << l) : r.tiles;
+}
+
+StartRoute start_route(const pa_params *prm, const GenPlan &plan)
+{
+    StartRoute r{};
+    const uint64_t nodes = plan.u_split - plan.u_first;
+    r.alone = plan.u_split >= prm->n && nodes > 0;
+    const double p = plan.model == PA_MODEL_BA ? 0.5 : prm->p;
+    r.variant = start_variant(nodes, prm->d, p);
+    const uint64_t slot_bytes = (plan.slots ? 1u : 2u) * plan.id_bytes;
+    if (r.alone && kCtlBytes + kHopBytes <= plan.start_offset &&
+        start_hops(nodes * prm->d * slot_bytes, p))
+        r.variant = {kStartMinBlocksMid, (uint32_t)kStartPasses, true};
+    r.tile_nodes = (uint64_t)r.variant.passes * plan.groups;
+    r.tiles = (nodes + r.tile_nodes - 1) / r.tile_nodes;
+    r.first_tiles = r.variant.hop ? std::min(r.tiles, kHopFirstNodes / r.tile_nodes) : r.tiles;
+    r.launches = nodes > 0 ? 1 : 0;
+    while (r.launches > 0 && tiles_after(r, r.launches - 1) < r.tiles) ++r.launches;
+    return r;
+}
+
+}  // namespace
+
+uint32_t generate_launches(const pa_params *prm, const GenPlan &plan)
+{
+    if (plan.wide) return 2;   // set-up, wide kernel
+    const StartRoute r = start_route(prm, plan);
+    if (r.alone) return 1 + r.launches;
+    // a seed-only graph stores nothing in SLOTS
+    return r.launches + (plan.slots && r.launches == 0 ? 0 : 1);
+}
+
 int launch_generate(const pa_params *prm, const GenPlan &plan, void *d_edges, void *d_scratch,
                     cudaStream_t stream, uint32_t blocks_override, const cudaEvent_t *events)
 {
@@ -466,7 +517,8 @@ int launch_generate(const pa_params *prm, const GenPlan &plan, void *d_edges, vo
     cudaError_t e = cudaSuccess;
     // every node by the start kernel or the wide kernel: no tile flags, superblock
     // counts or trace to clear
-    const bool alone = plan.wide || (plan.u_split >= prm->n && plan.u_split > plan.u_first);
+    const StartRoute route = plan.wide ? StartRoute{} : start_route(prm, plan);
+    const bool alone = plan.wide || route.alone;
     if (alone) {
         uint64_t off = 0, len = 0;
         if (!prefilled) fill_region(*prm, plan, &off, &len);
@@ -553,38 +605,25 @@ int launch_generate(const pa_params *prm, const GenPlan &plan, void *d_edges, vo
         sa.one = a;
         sa.count = 1;
         sa.write_seeds = 1;
-        const double p = plan.model == PA_MODEL_BA ? 0.5 : prm->p;
-        StartVariant variant = start_variant(plan.u_split - plan.u_first, prm->d, p);
-        // the filter and the launches' counters lie where tile flags would, unused here
-        constexpr uint64_t hop_bytes = kHopFilterBytes + kHopMaxLaunches * kStartAreaBytes;
-        const uint64_t slot_bytes = (plan.slots ? 1u : 2u) * plan.id_bytes;
-        if (alone && kCtlBytes + hop_bytes <= plan.start_offset &&
-            start_hops((plan.u_split - plan.u_first) * prm->d * slot_bytes, p))
-            variant = {kStartMinBlocksMid, (uint32_t)kStartPasses, true};
-        const uint64_t tile_nodes = (uint64_t)variant.passes * plan.groups;
-        sa.t_end = (plan.u_split - plan.u_first + tile_nodes - 1) / tile_nodes;
         sa.ticket = reinterpret_cast<unsigned long long *>(reinterpret_cast<unsigned char *>(d_scratch) +
                                                           plan.start_offset);
         sa.ctl = a.ctl;
         mrc = mark(1);
         if (mrc != PA_OK) return mrc;
-        const unsigned long long tiles = sa.t_end;
-        if (variant.hop) {
+        if (route.variant.hop) {
             unsigned char *spare = reinterpret_cast<unsigned char *>(d_scratch) + kCtlBytes;
-            e = cudaMemsetAsync(spare, 0, hop_bytes, stream);
+            e = cudaMemsetAsync(spare, 0, kHopBytes, stream);
             if (e != cudaSuccess) return set_cuda_error(e);
             sa.rejected = reinterpret_cast<uint32_t *>(spare);
             sa.ticket = reinterpret_cast<unsigned long long *>(spare + kHopFilterBytes);
-            sa.t_end = std::min<unsigned long long>(tiles, kHopFirstNodes / tile_nodes);
         }
-        for (uint32_t l = 1;; ++l) {
-            const int rc = launch_start(plan.id_bytes, sa, blocks, stream, plan.slots, variant);
+        for (uint32_t l = 0; l < route.launches; ++l) {
+            sa.t_end = tiles_after(route, l);
+            const int rc = launch_start(plan.id_bytes, sa, blocks, stream, plan.slots, route.variant);
             if (rc != PA_OK) return rc;
-            if (sa.t_end == tiles) break;
             sa.write_seeds = 0;
             sa.t_begin = sa.t_end;
-            sa.t_end = l + 1 < kHopMaxLaunches ? std::min(tiles, 2 * sa.t_end) : tiles;
-            sa.hop_end = (uint32_t)(plan.u_first + sa.t_begin * tile_nodes);
+            sa.hop_end = (uint32_t)(plan.u_first + sa.t_begin * route.tile_nodes);
             sa.ticket += kStartAreaBytes / sizeof(*sa.ticket);
         }
         if (plan.u_split >= prm->n) {

@@ -102,4 +102,7 @@ int launch_generate(const pa_params *prm, const GenPlan &plan, void *d_edges, vo
                     cudaStream_t stream, uint32_t blocks_override,
                     const cudaEvent_t *events = nullptr);
 
+// Kernels that launch_generate launches.
+uint32_t generate_launches(const pa_params *prm, const GenPlan &plan);
+
 }  // namespace pa

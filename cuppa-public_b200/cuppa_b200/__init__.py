@@ -171,6 +171,8 @@ _SIGS = {
     "pa_generate_finish": (ctypes.c_int, [ctypes.c_void_p, _P(PaStats), ctypes.c_void_p]),
     "pa_fill": (ctypes.c_int, [_P(PaParams), ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p]),
     "pa_start_split": (ctypes.c_int, [_P(PaParams), _P(ctypes.c_uint64)]),
+    "pa_generate_launches": (ctypes.c_int, [_P(PaParams), _P(ctypes.c_uint32)]),
+    "pa_csr_launches": (ctypes.c_int, [_P(PaParams), _P(ctypes.c_uint32)]),
     "pa_generate_timed": (ctypes.c_int, [_P(PaParams), ctypes.c_void_p, ctypes.c_uint64,
                                          ctypes.c_void_p, ctypes.c_uint64, ctypes.c_void_p,
                                          _P(ctypes.c_void_p)]),
@@ -373,6 +375,20 @@ def start_split(prm: PaParams) -> int:
     u = ctypes.c_uint64()
     check(lib().pa_start_split(ctypes.byref(prm), ctypes.byref(u)), "pa_start_split")
     return int(u.value)
+
+
+def generate_launches(prm: PaParams) -> int:
+    """Kernels that one generation launches (pa_generate_launches)."""
+    k = ctypes.c_uint32()
+    check(lib().pa_generate_launches(ctypes.byref(prm), ctypes.byref(k)), "pa_generate_launches")
+    return int(k.value)
+
+
+def csr_launches(prm: PaParams) -> int:
+    """Kernels that one CSR build launches (pa_csr_launches)."""
+    k = ctypes.c_uint32()
+    check(lib().pa_csr_launches(ctypes.byref(prm), ctypes.byref(k)), "pa_csr_launches")
+    return int(k.value)
 
 
 def finish(scratch, stream=None) -> PaStats:

@@ -142,6 +142,9 @@ int pa_scratch_bytes(const pa_params *prm, uint64_t *bytes);
  * rest by the persistent launch. */
 int pa_start_split(const pa_params *prm, uint64_t *u_split);
 
+/* Kernels that one pa_generate call launches (memory clears not counted). */
+int pa_generate_launches(const pa_params *prm, uint32_t *kernels);
+
 /* ---- generation ---------------------------------------------------------- */
 /* Stream-ordered generation into caller memory.  d_scratch (pa_scratch_bytes)
  * is cleared by the call; it must not be shared by generations that overlap.
@@ -236,6 +239,8 @@ int pa_digest(const void *d_ids, uint64_t count, uint32_t id_bits, uint64_t inde
  * Sizes of the three buffers: */
 int pa_csr_bytes(const pa_params *prm, uint64_t *rowptr_bytes, uint64_t *col_bytes,
                  uint64_t *scratch_bytes);
+/* Kernels that one pa_build_csr call launches (memory clears not counted). */
+int pa_csr_launches(const pa_params *prm, uint32_t *kernels);
 /* Builds the CSR on `stream` and waits for it (for its error word).  The in
  * parts come from a stable radix sort of the pairs by destination; the column
  * buffer doubles as sort space during the call.  d_col and d_scratch must be
