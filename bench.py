@@ -104,15 +104,17 @@ def load_peaks():
         return 6650.0, "fallback"
 
 
-def load_traffic(workload: str):
-    """Per-launch DRAM bytes of the dominant kernel from a committed ncu summary."""
+def load_traffic(workload: str, launches: int):
+    """DRAM bytes of the dominant kernel's launches in one generation, and where they come
+    from, by a committed ncu summary; (None, None) where it was taken over another number
+    of launches than now."""
     path = os.path.join(ROOT, "profiles", "kernel_traffic.json")
     try:
         with open(path) as f:
-            t = json.load(f)
-        return t.get(workload, {}).get("dram_bytes_per_launch")
+            t = json.load(f).get(workload, {})
+        return (t["dram_bytes"], t["source"]) if t.get("launches") == launches else (None, None)
     except Exception:
-        return None
+        return None, None
 
 
 def load_fixture_digests(name):
@@ -509,7 +511,8 @@ def run_gpu(args, w):
         else:
             kernel, k_edges, kern_s = "start_kernel", start_edges, statistics.mean(start_ms) / 1e3
         achieved = k_edges * bpe / kern_s / 1e9
-        traffic = load_traffic(args.workload)     # ncu DRAM bytes of one such launch
+        # ncu DRAM bytes of the kernel (its launches: all but the set-up kernel's)
+        traffic, traffic_source = load_traffic(args.workload, pa.generate_launches(prm) - 1)
         line = {
             "metric": w.get("metric", METRIC), "value": value, "unit": "edges/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms / args.steps,
@@ -523,6 +526,7 @@ def run_gpu(args, w):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak, "peak_source": peak_kind,
                          "bytes_per_edge": bpe, "traffic": traffic,
+                         "traffic_source": traffic_source,
                          # the DRAM the launch actually moves (whole 128-byte lines
                          # for random reads) over its measured time
                          "traffic_gbs": traffic / kern_s / 1e9 if traffic else None,
