@@ -85,18 +85,14 @@ constexpr uint32_t kDegChunk = 8192;   // pairs per block step at most
 constexpr uint64_t kDegNarrow = 1ull << 22;   // nodes above which 32-bit counts pay
 constexpr uint32_t kLowIds = 8192;     // 32 KB of shared counters
 
-// The counts before any pair is read: d out-edges of a generated node, and with `seeds`
-// the seed edges, both ends (CLIQUE: every seed node has d; STAR_REF: node d has d, the
-// others 1).
+// The counts before any pair is read: d from node `from` on, `low` below.
 template <typename Cnt>
-__global__ void __launch_bounds__(kDegThreads) degree_init_kernel(Cnt *deg, uint64_t n, uint64_t u_first,
-                                                                  uint32_t d, bool seeds,
-                                                                  uint32_t seed_mode)
+__global__ void __launch_bounds__(kDegThreads) degree_init_kernel(Cnt *deg, uint64_t n, uint64_t from,
+                                                                  uint32_t d, uint32_t low)
 {
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
-    const Cnt low = !seeds ? 0 : (seed_mode == PA_SEED_CLIQUE ? (Cnt)d : (Cnt)1);
     for (uint64_t u = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; u < n; u += stride)
-        deg[u] = u >= u_first || (seeds && u == d) ? (Cnt)d : low;
+        deg[u] = u >= from ? (Cnt)d : (Cnt)low;
 }
 
 // Pairs (or, with Slots, targets) of the generated nodes: `count` of them from E
@@ -294,8 +290,11 @@ template <typename Id, bool Slots, typename Cnt>
 void degrees_launch(const pa_params *prm, const GenPlan &p, const Id *E, Cnt *deg, cudaStream_t s)
 {
     const uint64_t n = prm->n, count = (n - p.u_first) * prm->d;
-    degree_init_kernel<Cnt><<<grid_for(n, kDegThreads), kDegThreads, 0, s>>>(deg, n, p.u_first, prm->d,
-                                                                             Slots, prm->seed_mode);
+    // the generated nodes' out-edges; with SLOTS the seed edges too, both ends (CLIQUE:
+    // every seed node has d; STAR_REF: node d has d, the others 1)
+    const uint64_t from = !Slots ? p.u_first : (prm->seed_mode == PA_SEED_CLIQUE ? 0 : prm->d);
+    degree_init_kernel<Cnt><<<grid_for(n, kDegThreads), kDegThreads, 0, s>>>(deg, n, from, prm->d,
+                                                                             Slots ? 1u : 0u);
     // floor(x / d) = umulhi(x, d_inv) for x below 2^16: d_inv = ceil(2^32 / d) is off
     // by less than 1 / x (d = 1: 2^32 does not fit)
     // one load per pair when the pairs are aligned to their size
