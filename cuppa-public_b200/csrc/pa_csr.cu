@@ -23,10 +23,9 @@
 // and each pass is one kernel that keeps its tile on chip from the load to the
 // store, taking each digit's offset from the tiles before it by decoupled
 // look-back (Merrill and Garland's single-pass prefix scan, as in Adinets and
-// Merrill's one-sweep radix sort) instead of a per-pass histogram and scan.
+// Merrill's one-sweep radix sort) instead of a per-pass histogram and scan.  Ranks come
+// from lane masks that equal digits collect in shared memory, as public radix sorts do.
 #include <algorithm>
-#include <type_traits>
-#include <vector>
 
 #include "pa_device.cuh"
 #include "pa_internal.h"
@@ -141,11 +140,11 @@ __global__ void __launch_bounds__(kRadixThreads) radix_hist_all_kernel(const Id 
     __syncthreads();
     constexpr uint32_t U = 4;   // items per thread per step, loaded together
     const uint64_t stride = (uint64_t)gridDim.x * kRadixThreads * U;
-    for (uint64_t base = (uint64_t)blockIdx.x * kRadixThreads * U; base < n_items; base += stride) {
+    for (uint64_t i0 = (uint64_t)blockIdx.x * kRadixThreads * U; i0 < n_items; i0 += stride) {
         uint32_t key[U];
 #pragma unroll
         for (uint32_t j = 0; j < U; ++j) {
-            const uint64_t i = base + j * kRadixThreads + threadIdx.x;
+            const uint64_t i = i0 + j * kRadixThreads + threadIdx.x;
             key[j] = 0u;
             if (i < n_items) {
                 const unsigned long long it = pair_item(E, i, n, err);
@@ -155,7 +154,7 @@ __global__ void __launch_bounds__(kRadixThreads) radix_hist_all_kernel(const Id 
         }
 #pragma unroll
         for (uint32_t j = 0; j < U; ++j) {
-            if (base + j * kRadixThreads + threadIdx.x >= n_items) continue;
+            if (i0 + j * kRadixThreads + threadIdx.x >= n_items) continue;
             for (uint32_t q = 0; q < passes; ++q)
                 atomicAdd(&cnt[q * NB + ((key[j] >> (DB * q)) & MASK)], 1u);
         }
@@ -208,8 +207,8 @@ struct RadixSmem {
     unsigned long long tile;
 };
 
-// What bounds it: the shared-memory pipe (77 % busy in a capture at 9.6 * 10^7
-// items; DRAM 27 %), ~52 wavefronts per 32 items.  __match_any_sync for the
+// What bounds it: the load/store data pipe, mostly its shared-memory half (75 % busy in
+// a capture at 4.8 * 10^7 items; DRAM 26 %), ~52 wavefronts per 32 items.  __match_any_sync for the
 // equal digits, which the words replace, costs two cycles of a unit shared by
 // the SM per distinct value: 61 cycles a round of 32 mostly distinct digits
 // against 7.5 for the atomicOr, the word's load and its store (measured alone).
@@ -493,7 +492,7 @@ __global__ void in_sorted_kernel(const unsigned long long *items, uint64_t n_ite
 // more, by shuffles within the 32 positions that hold them (five steps instead of
 // eight, no bank conflicts): n = 2.5 * 10^7, d = 16: 1.25 ms by shuffles alone, now 0.72; n =
 // 2^27, d = 4, p = 0.1, the whole CSR: 20.3 ms by shuffles alone, 22.5 in shared memory
-// alone, now 18.3.
+// alone, 18.3 so (17.9 with the row writer's registers unspilled).
 constexpr uint64_t kRowWeight = 4;
 constexpr uint32_t kFewRows = 64;
 constexpr uint32_t kRowSpan = 256;
@@ -996,7 +995,7 @@ int csr_enqueue_t(const pa_params *prm, const GenPlan &p, const Id *E, int64_t *
                         : (unsigned long long *)(scratch + L.status_off);
     if (m > 0) {
         int rc = PA_ERR_INVALID;
-        // small tiles where tiles of 8,192 would leave SMs idle (n = 2 * 10^4, d = 6:
+        // small tiles where tiles of 8,192 would leave some of the 148 SMs idle (n = 2 * 10^4, d = 6:
         // 15 of them; a pass 11.5 -> 8.9 us), if their look-back words -- four times as many
         // -- fit the column buffer's half or the row starts, not written yet
         constexpr uint64_t kSmallTile = kRadixThreads * kRadixRoundsSmall;

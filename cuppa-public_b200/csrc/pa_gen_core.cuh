@@ -65,7 +65,8 @@ inline StartVariant start_variant(uint64_t start_nodes, uint32_t d, double p)
 // slots are ever rejected.  Without -> with, ms (64-bit ids, d = 4 unless given):
 //  * n = 2^28, p = 0.5 15.82 -> 13.92, 0.4 18.36 -> 16.60, 0.6 14.12 -> 13.30; with fewer
 //    copies the draws cost more than the reads (0.7 11.69 -> 12.35), with more of
-//    them most are of copies (0.25 20.94 -> 20.44);
+//    them most are of copies (0.25 20.94 -> 20.44).  The lines lie at the last points
+//    with a clear gain; p between them and those beyond was not measured;
 //  * 2.1 GB, n = 2^25: 1.97 -> 1.86; 4.3 GB 3.90 -> 3.56, d = 8 4.03 -> 3.68; SLOTS 2.1 GB
 //    3.18 -> 3.05; 32-bit ids 8.6 GB 13.42 -> 12.26, d = 32 13.68 -> 12.81; below, the
 //    second-level cache answers more of the reads (1.6 GB, d = 5: 1.47 -> 1.50; 1 GB,

@@ -526,6 +526,7 @@ int launch_generate(const pa_params *prm, const GenPlan &plan, void *d_edges, vo
         unsigned char *edges = reinterpret_cast<unsigned char *>(d_edges);
         const bool small = len <= kPrepareBytes;
         const uint64_t blocks16 = small ? (len / 16 + 255) / 256 : 0;
+        // eight blocks a SM (148) at most
         prepare_kernel<<<(unsigned)std::max<uint64_t>(1, std::min<uint64_t>(blocks16, 148 * 8)), 256, 0,
                          stream>>>(reinterpret_cast<uint4 *>(scr), kCtlBytes / 16,
                                    reinterpret_cast<uint4 *>(scr + plan.start_offset),

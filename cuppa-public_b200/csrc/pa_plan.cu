@@ -1,8 +1,8 @@
 // pa_plan.cu -- a generation captured once into a CUDA graph and replayed.
 //
 // A small graph (10^4..10^5 nodes) takes tens of microseconds on the GPU, the
-// same order as issuing its scratch clear, sentinel fill and kernel launch one
-// by one.  A plan records that sequence for fixed parameters and buffers with
+// same order as issuing its launches (set-up and start kernel; clears, fills and more
+// launches in larger graphs) one by one.  A plan records that sequence for fixed parameters and buffers with
 // stream capture and replays it with one cudaGraphLaunch.  The replay writes
 // exactly what pa_generate writes (the captured work is pa_generate's).
 #include <new>

@@ -3,7 +3,7 @@
 // One graph never spans GPUs: every copy read may land on any earlier node, so
 // a graph stays on the GPU that generates it, and more GPUs serve more graphs.
 // The router owns one request server per device (pa_server_*, each with its own
-// control thread, memory pool and admission queue) and places each request on
+// control threads, memory and admission queue) and places each request on
 // the server whose routed, unreleased bytes would be the smallest fraction of
 // its budget.  Tickets carry the server index in their low byte; results, waits
 // and releases go to that server.  No data crosses between GPUs, so there is no

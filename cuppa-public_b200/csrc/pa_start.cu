@@ -11,7 +11,8 @@
 // poll round trip, the first few million nodes of a graph cost milliseconds.
 //
 // This kernel takes the tile out of the chain.  Before it runs, every pair of
-// its region is set to all-ones (a memset), which is never a node id.  A lane
+// its region is set to all-ones (by the set-up kernel, a memset above 32 MB), which is
+// never a node id.  A lane
 // stores its slot's pair the moment the slot is final -- every lower slot of
 // its node final and its candidate distinct from theirs -- and a copy read of
 // slot (v, k) re-reads that pair's target field until it is not all-ones.  The
@@ -21,7 +22,7 @@
 // warp pass are taken from the source lane by shuffle once it is final, as in
 // the persistent kernel.  (Filling inside the kernel instead -- each warp
 // filling the tile it claims, with per-tile opened flags and a watermark for
-// readers -- measured slower on B200 than the memset it saves: 88.7 against
+// readers -- measured slower on B200 than the fill it saves: 88.7 against
 // 68.0 ms for n = 2^30, d = 4.)
 //
 // Work is claimed one start tile at a time: P warp passes (1, 2 or kStartPasses,

@@ -519,7 +519,8 @@ def write_edges(prm: PaParams, edges, path: str, binary: bool = False, stream=No
 # Edges per chunk handed to a Python sink: its bytes objects (~1 MB of text) come
 # from memory that malloc keeps, where those of the library's 2^24-edge chunks are
 # mapped and faulted in anew each time (n = 10^6, d = 4: 28.2 -> 6.8 ms; n = 2 * 10^6,
-# d = 16: 230 -> 57 ms; 2^18 edges: 7.5 and 64 ms).
+# d = 16: 230 -> 57 ms; 2^18 edges: 7.5 and 64 ms; binary, n = 10^6, d = 4: 4.2 -> 2.3
+# ms, d = 16: 59 -> 7.5).
 _SINK_CHUNK_EDGES = 1 << 16
 
 _SINK = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint64)
@@ -528,9 +529,9 @@ _SINK = ctypes.CFUNCTYPE(ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.
 def stream_edges(prm: PaParams, edges, sink, binary: bool = False, chunk_edges: int = 0,
                  stream=None) -> int:
     """pa_stream_edges: sink(bytes) receives the output in order (called from a
-    library thread), about chunk_edges edges (0: 2^16) at a time, whole rows; returns
-    the byte count.  A sink that raises or returns a true value stops the stream
-    (PaError PA_ERR_IO)."""
+    library thread), about chunk_edges edges (0: 2^16, where the C entry takes 2^24) at a
+    time, whole rows; returns the byte count.  A sink that raises or returns a
+    true value stops the stream (CuppaError PA_ERR_IO)."""
     def _cb(ctx, data, nbytes):
         try:
             return 1 if sink(ctypes.string_at(data, nbytes)) else 0

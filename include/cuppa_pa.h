@@ -423,8 +423,9 @@ typedef int (*pa_sink_fn)(void *ctx, const void *data, uint64_t bytes);
  * (src/PA/SPA/PAHelper.hpp:163-177; with PA_SEED_STAR_REF also its row order);
  * BINARY = little-endian (src, dst) id pairs of id_bits each.  Order: the seed
  * edges, then rows u = d+1..n-1 in slot order.  The text is formatted on the
- * device; chunks of about chunk_edges edges (0 = 2^24) are copied to pinned host
- * memory while the next chunk is formatted and the previous one is sunk.  Runs
+ * device; chunks of about chunk_edges edges (0 = 2^24; the Python binding's default
+ * is 2^16) are copied to pinned host memory while the next chunk is formatted and
+ * the previous one is sunk.  Runs
  * after the work already queued on `stream`; waits.  *bytes_out (optional) gets
  * the byte count. */
 int pa_stream_edges(const pa_params *prm, const void *d_edges, int format, uint64_t chunk_edges,
